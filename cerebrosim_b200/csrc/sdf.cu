@@ -4,7 +4,8 @@
 // Per voxel p = origin + (i, j, k) dx: for each branch, the minimum over its segments of the round-cone distance
 // |p - (a + t ab)| - r(t) (t = the clamped projection of p on the segment, r interpolated linearly), cut by the flat
 // caps near its open ends (a half-space max within 2.5 cap radii); branches are joined by the polynomial smooth
-// minimum with blend radius `blend`. Negative inside the lumen. One thread per voxel, C order (k fastest).
+// minimum with blend radius `blend`. Negative inside the lumen. One thread per voxel, C order (k fastest); a block
+// works a brick of voxels with the segments that can be nearest there.
 #include "cs_common.cuh"
 
 namespace cs {
@@ -32,28 +33,142 @@ __device__ __forceinline__ float smin(float a, float b, float k) {
     return b + (a - b) * h - k * h * (1.0f - h);
 }
 
-__global__ void k_sdf(const SdfArgs s) {
-    const int64_t total = s.nx * s.ny * s.nz;
-    for (int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; c < total; c += int64_t(gridDim.x) * blockDim.x) {
-        const int64_t l = c % s.nz, j = (c / s.nz) % s.ny, i = c / (s.ny * s.nz);
+// Bricks of 8 x 4 x 8 voxels, one block of 256 threads each. Evaluating every segment at every voxel is bound by
+// instruction issue (about 45 per segment, the division and the square root among them; 330 segments on a vessel of
+// two branches), so a block first drops the segments that cannot be the nearest anywhere in its brick and a thread
+// then skips those of the rest that cannot beat the distance it already has. Only evaluations whose result the
+// minimum would discard are left out, so the field is the same bit for bit.
+//
+// Bounds, for a segment k with axis distance D_k(c) from the brick's centre c, brick half-diagonal h, and the radii
+// r0, r1 at its ends: anywhere in the brick |p - q| - r lies in [D_k(c) - h - max(r0, r1), D_k(c) + h - min(r0, r1)]
+// (a distance to a segment changes by at most the way walked). A segment whose lower end lies above the least upper
+// end U of all segments of its branch is never the minimum. For a voxel p and a segment of half-length l and midpoint
+// m, |p - q| >= |p - m| - l. Each bound carries a margin of 1e-5 of the lengths that enter it, over a hundred times
+// the rounding of its own evaluation and of the distances it is compared with. A comparison with NaN keeps the segment.
+constexpr int BX = 8, BY = 4, BZ = 8;
+constexpr int SDF_THREADS = BX * BY * BZ;
+constexpr float SDF_MARGIN = 1.0e-5f;
+
+// Axis distance of point c from segment k of the packed centrelines.
+__device__ __forceinline__ float axis_distance(const SdfArgs& s, int k, float cx, float cy, float cz) {
+    const float ax = __ldg(s.pts + 3 * k), ay = __ldg(s.pts + 3 * k + 1), az = __ldg(s.pts + 3 * k + 2);
+    const float bx = __ldg(s.pts + 3 * k + 3) - ax, by = __ldg(s.pts + 3 * k + 4) - ay, bz = __ldg(s.pts + 3 * k + 5) - az;
+    const float qx = cx - ax, qy = cy - ay, qz = cz - az;
+    const float t = fminf(fmaxf((qx * bx + qy * by + qz * bz) / fmaxf(bx * bx + by * by + bz * bz, 1.0e-12f), 0.0f), 1.0f);
+    const float ex = qx - bx * t, ey = qy - by * t, ez = qz - bz * t;
+    return sqrtf(ex * ex + ey * ey + ez * ez);
+}
+
+// vessel.py:195-199: distance of p to the round cone from a along b with radius r0 + dr t.
+__device__ __forceinline__ float cone_distance(float px, float py, float pz, float ax, float ay, float az, float bx,
+                                               float by, float bz, float r0, float dr) {
+    const float qx = px - ax, qy = py - ay, qz = pz - az;
+    const float t = fminf(fmaxf((qx * bx + qy * by + qz * bz) / fmaxf(bx * bx + by * by + bz * bz, 1.0e-12f), 0.0f), 1.0f);
+    const float r = r0 + dr * t;
+    const float ex = px - (ax + bx * t), ey = py - (ay + by * t), ez = pz - (az + bz * t);
+    return sqrtf(ex * ex + ey * ey + ez * ez) - r;
+}
+
+__global__ void __launch_bounds__(SDF_THREADS) k_sdf(const SdfArgs s, const int64_t nbx, const int64_t nby,
+                                                     const int64_t nbz) {
+    __shared__ float4 s_seg[2][SDF_THREADS];   // start and r0; direction and r1 - r0
+    __shared__ float4 s_mid[SDF_THREADS];      // midpoint; half-length + larger radius + margin
+    __shared__ float s_u[SDF_THREADS / 32];
+    __shared__ int s_cnt[SDF_THREADS / 32 + 1], s_best;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t bricks = nbx * nby * nbz;
+    for (int64_t br = blockIdx.x; br < bricks; br += gridDim.x) {
+        const int64_t z0 = (br % nbz) * BZ, y0 = ((br / nbz) % nby) * BY, x0 = (br / (nbz * nby)) * BX;
+        const int64_t l = z0 + tid % BZ, j = y0 + (tid / BZ) % BY, i = x0 + tid / (BZ * BY);
         const float px = s.origin[0] + float(i) * s.dx;
         const float py = s.origin[1] + float(j) * s.dx;
         const float pz = s.origin[2] + float(l) * s.dx;
+        const float cx = s.origin[0] + (float(x0) + 0.5f * float(BX - 1)) * s.dx;
+        const float cy = s.origin[1] + (float(y0) + 0.5f * float(BY - 1)) * s.dx;
+        const float cz = s.origin[2] + (float(z0) + 0.5f * float(BZ - 1)) * s.dx;
+        const float h = 0.5f * s.dx * sqrtf(float((BX - 1) * (BX - 1) + (BY - 1) * (BY - 1) + (BZ - 1) * (BZ - 1)));
+        const float size = fabsf(cx) + fabsf(cy) + fabsf(cz) + 4.0f * h;     // of the coordinates in the brick
         float d = 1.0e9f;
         for (int b = 0; b < s.nbranch; ++b) {
+            const int s0 = __ldg(s.br_start + b), last = s0 + __ldg(s.br_count + b) - 1;
+            // least upper bound over the branch's segments, and the segment that has it
+            float u_own = 3.0e38f;
+            int k_own = -1;
+            for (int k = s0 + tid; k < last; k += SDF_THREADS) {
+                const float dk = axis_distance(s, k, cx, cy, cz), r0 = __ldg(s.rad + k), r1 = __ldg(s.rad + k + 1);
+                const float up = dk + h - fminf(r0, r1) + SDF_MARGIN * (size + dk + fmaxf(fabsf(r0), fabsf(r1)));
+                if (up < u_own) {
+                    u_own = up;
+                    k_own = k;
+                }
+            }
+            float u = u_own;
+            for (int o = 16; o > 0; o >>= 1) u = fminf(u, __shfl_xor_sync(0xffffffffu, u, o));
+            if (lane == 0) s_u[warp] = u;
+            if (tid == 0) s_best = -1;
+            __syncthreads();
+            for (int w = 0; w < SDF_THREADS / 32; ++w) u = fminf(u, s_u[w]);
+            if (k_own >= 0 && u_own == u) s_best = k_own;      // of several, any
+            __syncthreads();
+            // the brick's nearest segment first: most of the others then fall to the test of their midpoint
             float db = 1.0e9f;
-            const int s0 = __ldg(s.br_start + b), cnt = __ldg(s.br_count + b);
-            for (int k = s0; k < s0 + cnt - 1; ++k) {
+            if (s_best >= 0) {
+                const int k = s_best;
                 const float ax = __ldg(s.pts + 3 * k), ay = __ldg(s.pts + 3 * k + 1), az = __ldg(s.pts + 3 * k + 2);
-                const float bx = __ldg(s.pts + 3 * k + 3) - ax, by = __ldg(s.pts + 3 * k + 4) - ay,
-                            bz = __ldg(s.pts + 3 * k + 5) - az;
-                const float qx = px - ax, qy = py - ay, qz = pz - az;
-                const float t = fminf(fmaxf((qx * bx + qy * by + qz * bz) / fmaxf(bx * bx + by * by + bz * bz, 1.0e-12f),
-                                            0.0f), 1.0f);
                 const float r0 = __ldg(s.rad + k);
-                const float r = r0 + (__ldg(s.rad + k + 1) - r0) * t;
-                const float ex = px - (ax + bx * t), ey = py - (ay + by * t), ez = pz - (az + bz * t);
-                db = fminf(db, sqrtf(ex * ex + ey * ey + ez * ez) - r);
+                db = fminf(db, cone_distance(px, py, pz, ax, ay, az, __ldg(s.pts + 3 * k + 3) - ax,
+                                             __ldg(s.pts + 3 * k + 4) - ay, __ldg(s.pts + 3 * k + 5) - az, r0,
+                                             __ldg(s.rad + k + 1) - r0));
+            }
+            for (int k0 = s0; k0 < last; k0 += SDF_THREADS) {
+                // the segments of this chunk that may be the nearest, kept in their order in shared memory
+                const int k = k0 + tid;
+                bool keep = false;
+                float r0 = 0.0f, r1 = 0.0f, dk = 0.0f;
+                if (k < last) {
+                    dk = axis_distance(s, k, cx, cy, cz);
+                    r0 = __ldg(s.rad + k);
+                    r1 = __ldg(s.rad + k + 1);
+                    const float rm = fmaxf(r0, r1);
+                    keep = !(dk - h - rm - SDF_MARGIN * (size + dk + fmaxf(fabsf(r0), fabsf(r1))) > u);
+                }
+                const unsigned mask = __ballot_sync(0xffffffffu, keep);
+                if (lane == 0) s_cnt[warp] = __popc(mask);
+                __syncthreads();
+                if (tid == 0) {
+                    int run = 0;
+                    for (int w = 0; w < SDF_THREADS / 32; ++w) {
+                        const int c = s_cnt[w];
+                        s_cnt[w] = run;
+                        run += c;
+                    }
+                    s_cnt[SDF_THREADS / 32] = run;
+                }
+                __syncthreads();
+                if (keep) {
+                    const int o = s_cnt[warp] + __popc(mask & ((1u << lane) - 1u));
+                    const float ax = __ldg(s.pts + 3 * k), ay = __ldg(s.pts + 3 * k + 1), az = __ldg(s.pts + 3 * k + 2);
+                    const float bx = __ldg(s.pts + 3 * k + 3) - ax, by = __ldg(s.pts + 3 * k + 4) - ay,
+                                bz = __ldg(s.pts + 3 * k + 5) - az;
+                    const float half = 0.5f * sqrtf(bx * bx + by * by + bz * bz);
+                    s_seg[0][o] = make_float4(ax, ay, az, r0);
+                    s_seg[1][o] = make_float4(bx, by, bz, r1 - r0);
+                    s_mid[o] = make_float4(ax + 0.5f * bx, ay + 0.5f * by, az + 0.5f * bz,
+                                           half + fmaxf(r0, r1) +
+                                               SDF_MARGIN * (size + dk + half + fmaxf(fabsf(r0), fabsf(r1))));
+                }
+                __syncthreads();
+                const int cnt = s_cnt[SDF_THREADS / 32];
+                for (int c = 0; c < cnt; ++c) {
+                    const float4 m = s_mid[c];
+                    const float gx = px - m.x, gy = py - m.y, gz = pz - m.z;
+                    // |p - m| - reach >= db: the distance below cannot be smaller than db
+                    const float far = (db + m.w) * 1.00001f;
+                    if (far < 0.0f || gx * gx + gy * gy + gz * gz > far * far) continue;
+                    const float4 a = s_seg[0][c], e = s_seg[1][c];
+                    db = fminf(db, cone_distance(px, py, pz, a.x, a.y, a.z, e.x, e.y, e.z, a.w, e.w));
+                }
+                __syncthreads();                    // the list is rewritten by the next chunk or branch
             }
             for (int e = 0; e < 2; ++e) {
                 const int cc = b * 2 + e;
@@ -67,8 +182,9 @@ __global__ void k_sdf(const SdfArgs s) {
                 }
             }
             d = smin(d, db, s.blend);
+            __syncthreads();                        // s_u is rewritten by the next branch
         }
-        s.out[c] = d;
+        if (i < s.nx && j < s.ny && l < s.nz) s.out[(i * s.ny + j) * s.nz + l] = d;
     }
 }
 
@@ -90,8 +206,9 @@ extern "C" int cs_sdf_vessel(const float* pts, const float* rad, const int32_t* 
         return fail(CS_ERR_ARG, "cs_sdf_vessel: null buffer");
     SdfArgs a{{origin[0], origin[1], origin[2]}, dx, pts, rad, br_start, br_count, cap_p, cap_n, cap_r, blend,
               nbranch, nx, ny, nz, out};
-    const unsigned grid = unsigned(std::min<int64_t>(ceil_div(total, 256), 148 * 64));
-    k_sdf<<<grid, 256, 0, as_stream(stream)>>>(a);
+    const int64_t nbx = ceil_div(nx, BX), nby = ceil_div(ny, BY), nbz = ceil_div(nz, BZ);
+    const unsigned grid = unsigned(std::min<int64_t>(nbx * nby * nbz, 148 * 64));
+    k_sdf<<<grid, SDF_THREADS, 0, as_stream(stream)>>>(a, nbx, nby, nbz);
     CS_CHECK_LAUNCH("k_sdf");
     return CS_OK;
 }

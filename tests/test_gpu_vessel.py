@@ -58,3 +58,30 @@ def test_empty_and_invalid_vessels(golden):
     empty = vessel.Packed([], np.zeros((0, 3)), np.zeros(0), [], [], np.zeros((0, 3)), np.zeros((0, 3)), [])
     phi, _ = vessel.sdf_grid(empty, 1.0, [0, 0, 0], [2, 3, 4])
     assert phi.shape == (3, 4, 5) and (phi == np.float32(1e9)).all()
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (8, 4, 8), (9, 5, 9), (7, 3, 17), (33, 18, 41)])
+@pytest.mark.parametrize("points", [(1, 2), (257, 3), (600, 700)])
+def test_sdf_bricks(shape, points):
+    """Voxel bricks with remainders on every axis; branches without a segment, of one chunk of 256 segments and of
+    several; a narrowing and a bend, so that the nearest segment changes inside a brick. Against the oracle's field
+    within the rounding of distances of coordinates up to 12 (an ulp of 9.5e-7, a dozen operations)."""
+    pts, rad = [], []
+    for b, n in enumerate(points):
+        t = np.linspace(0.0, 1.0, n)
+        pts.append(np.column_stack([9 * t, 2 * np.sin(5 * t + b), 6 * b * t + np.cos(3 * t)]))
+        rad.append(1.2 - 0.8 * np.exp(-((t - 0.5) / 0.05) ** 2))
+    start = np.cumsum([0] + [len(p) for p in pts[:-1]])
+    cap_p = np.concatenate([[p[0], p[-1]] for p in pts])
+    cap_n = np.tile([[-1.0, 0.0, 0.0], [1.0, 0.0, 0.0]], (len(pts), 1))
+    pk = vessel.Packed(["a", "b"], np.concatenate(pts), np.concatenate(rad), start, points, cap_p, cap_n,
+                       [1.2, 0.0, 0.0, 1.2])
+    dx = 0.31
+    lo = np.array([-1.5, -2.5, -1.5])
+    hi = lo + (np.array(shape) - 1.5) * dx
+    gpu, _ = vessel.sdf_grid(pk, dx, lo, hi)
+    ref = sdf_ref.sdf_grid(pk.arrays(), lo, hi, dx)
+    assert gpu.shape == tuple(max(1, n) for n in shape) == ref.shape
+    both = np.abs(ref) < 1e8                              # a vessel without a segment stays at its initial 1e9
+    assert ((np.abs(gpu) < 1e8) == both).all()
+    assert np.abs(gpu.astype(np.float64) - ref)[both].max(initial=0.0) <= 2e-5
