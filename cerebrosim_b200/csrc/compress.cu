@@ -83,31 +83,8 @@ __global__ void k_cmp_count(const uint8_t* __restrict__ flags, int64_t n, int64_
 }
 
 // Exclusive scan of one flag's tile counts (block b: 0 irregular, 1 segment starts); totals at part[b][tiles].
-__global__ void k_cmp_scan(int64_t* __restrict__ part, int64_t tiles) {
-    __shared__ int64_t s[1024];
-    int64_t* p = part + int64_t(blockIdx.x) * (tiles + 1);
-    const int64_t per = ceil_div(tiles, blockDim.x);
-    const int64_t lo = threadIdx.x * per, hi = min(lo + per, tiles);
-    int64_t sum = 0;
-    for (int64_t t = lo; t < hi; ++t) sum += p[t];
-    s[threadIdx.x] = sum;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int64_t run = 0;
-        for (int k = 0; k < (int)blockDim.x; ++k) {
-            const int64_t x = s[k];
-            s[k] = run;
-            run += x;
-        }
-        p[tiles] = run;
-    }
-    __syncthreads();
-    int64_t run = s[threadIdx.x];
-    for (int64_t t = lo; t < hi; ++t) {
-        const int64_t x = p[t];
-        p[t] = run;
-        run += x;
-    }
+__global__ void __launch_bounds__(1024) k_cmp_scan(int64_t* __restrict__ part, int64_t tiles) {
+    block_exclusive_scan(part + int64_t(blockIdx.x) * (tiles + 1), tiles);
 }
 
 __global__ void k_cmp_fill(const int32_t* __restrict__ links, const uint8_t* __restrict__ flags, int64_t n,

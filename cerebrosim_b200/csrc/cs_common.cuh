@@ -53,6 +53,41 @@ constexpr int32_t WALL_TAG_LIMIT = -(1 << 30);
 __host__ __device__ inline bool is_wall(int32_t code) { return code < WALL_TAG_LIMIT; }
 __device__ inline float wall_q(int32_t code) { return __int_as_float(code & 0x7fffffff); }
 
+// Exclusive scan of p[0 .. n) in place by one block of 1024 threads; p[n] receives the total. Each thread sums a run
+// of its own, the runs are scanned by shuffles (a serial loop of one thread over 1024 partial sums took 9 us).
+__device__ inline void block_exclusive_scan(int64_t* __restrict__ p, int64_t n) {
+    __shared__ int64_t s_warp[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t per = (n + blockDim.x - 1) / blockDim.x;
+    const int64_t lo = min(int64_t(threadIdx.x) * per, n), hi = min(lo + per, n);
+    int64_t sum = 0;
+    for (int64_t t = lo; t < hi; ++t) sum += p[t];
+    int64_t run = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int64_t v = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += v;
+    }
+    if (lane == 31) s_warp[warp] = run;
+    __syncthreads();
+    if (warp == 0) {
+        int64_t w = s_warp[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t v = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += v;
+        }
+        s_warp[lane] = w;
+    }
+    __syncthreads();
+    run += (warp ? s_warp[warp - 1] : 0) - sum;
+    for (int64_t t = lo; t < hi; ++t) {
+        const int64_t v = p[t];
+        p[t] = run;
+        run += v;
+    }
+    if (threadIdx.x == 0) p[n] = s_warp[31];
+    __syncthreads();
+}
+
 // ---- error reporting (per host thread) ------------------------------------------------------------------------
 void set_error(const char* fmt, ...);
 int fail(int code, const char* fmt, ...);

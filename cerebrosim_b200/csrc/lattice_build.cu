@@ -20,6 +20,12 @@ constexpr int TILE_THREADS = 256;
 constexpr int TILE_ROUNDS = 16;
 constexpr int64_t TILE = TILE_THREADS * TILE_ROUNDS;
 constexpr int MAX_OPENINGS = 32;
+constexpr uint32_t INLET_CELL = 1u;      // in a node's first profile word, between pass B and the profile itself
+
+__constant__ int8_t k_c[3][Q] = {
+    {0, 1, -1, 0, 0, 0, 0, 1, -1, 1, -1, 1, -1, 1, -1, 0, 0, 0, 0, 1, -1, 1, -1, 1, -1, -1, 1},
+    {0, 0, 0, 1, -1, 0, 0, 1, -1, -1, 1, 0, 0, 0, 0, 1, -1, 1, -1, 1, -1, 1, -1, -1, 1, 1, -1},
+    {0, 0, 0, 0, 0, 1, -1, 0, 0, 0, 0, 1, -1, -1, 1, 1, -1, -1, 1, 1, -1, -1, 1, 1, -1, 1, -1}};
 
 struct ScratchLayout {
     int64_t n_tiles;
@@ -58,66 +64,50 @@ __global__ void k_tile_count(const float* __restrict__ phi, int64_t m, int64_t* 
 }
 
 // Exclusive scan of the tile counts by one block (tile_cnt[n_tiles] receives the total).
-__global__ void k_tile_scan(int64_t* __restrict__ tile_cnt, int64_t n_tiles, int64_t* __restrict__ n_fluid) {
-    __shared__ int64_t part[1024];
-    int64_t per = ceil_div(n_tiles, blockDim.x);
-    int64_t lo = threadIdx.x * per, hi = min(lo + per, n_tiles);
-    int64_t s = 0;
-    for (int64_t t = lo; t < hi; ++t) s += tile_cnt[t];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int64_t run = 0;
-        for (int k = 0; k < (int)blockDim.x; ++k) {
-            int64_t v = part[k];
-            part[k] = run;
-            run += v;
-        }
-        *n_fluid = run;
-        tile_cnt[n_tiles] = run;
-    }
-    __syncthreads();
-    int64_t run = part[threadIdx.x];
-    for (int64_t t = lo; t < hi; ++t) {
-        int64_t v = tile_cnt[t];
-        tile_cnt[t] = run;
-        run += v;
-    }
+__global__ void __launch_bounds__(1024) k_tile_scan(int64_t* __restrict__ tile_cnt, int64_t n_tiles, int64_t* __restrict__ n_fluid) {
+    block_exclusive_scan(tile_cnt, n_tiles);
+    if (threadIdx.x == 0) *n_fluid = tile_cnt[n_tiles];
 }
 
+// Each warp ranks TILE_ROUNDS consecutive groups of 32 cells: all its loads are issued before the first ballot, and
+// the block meets once (a barrier per group of 256 cells took 16 us on a grid of 2.8 M cells, this takes 5).
 __global__ void k_tile_rank(const float* __restrict__ phi, int64_t m, const int64_t* __restrict__ tile_off,
                             int32_t* __restrict__ rank) {
     __shared__ int warp_cnt[TILE_THREADS / 32];
-    __shared__ int64_t run;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) run = tile_off[blockIdx.x];
-    int64_t base = int64_t(blockIdx.x) * TILE;
+    const int64_t base = int64_t(blockIdx.x) * TILE + int64_t(warp) * (32 * TILE_ROUNDS) + lane;
+    float v[TILE_ROUNDS];
+#pragma unroll
+    for (int r = 0; r < TILE_ROUNDS; ++r) v[r] = base + 32 * r < m ? phi[base + 32 * r] : 0.0f;
+    unsigned mask[TILE_ROUNDS];
+    int total = 0;
+#pragma unroll
     for (int r = 0; r < TILE_ROUNDS; ++r) {
-        int64_t c = base + int64_t(r) * TILE_THREADS + threadIdx.x;
-        bool fl = c < m && phi[c] < 0.0f;
-        unsigned mask = __ballot_sync(0xffffffffu, fl);
-        if (lane == 0) warp_cnt[warp] = __popc(mask);
-        __syncthreads();
-        int64_t before = run;
-        for (int w = 0; w < warp; ++w) before += warp_cnt[w];
-        if (c < m) rank[c] = fl ? int32_t(before + __popc(mask & ((1u << lane) - 1u))) : -1;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int64_t t = 0;
-            for (int w = 0; w < TILE_THREADS / 32; ++w) t += warp_cnt[w];
-            run += t;
-        }
-        __syncthreads();
+        mask[r] = __ballot_sync(0xffffffffu, v[r] < 0.0f);
+        total += __popc(mask[r]);
+    }
+    if (lane == 0) warp_cnt[warp] = total;
+    __syncthreads();
+    int64_t before = tile_off[blockIdx.x];
+    for (int w = 0; w < warp; ++w) before += warp_cnt[w];
+#pragma unroll
+    for (int r = 0; r < TILE_ROUNDS; ++r) {
+        if (base + 32 * r < m)
+            rank[base + 32 * r] = (mask[r] >> lane) & 1u ? int32_t(before + __popc(mask[r] & ((1u << lane) - 1u))) : -1;
+        before += __popc(mask[r]);
     }
 }
 
+// IDX: int32_t when the grid has fewer than 2^31 cells (a 64-bit division is a subroutine of some 70 instructions).
+template <class IDX>
 __global__ void k_coords(const int32_t* __restrict__ rank, int64_t nx, int64_t ny, int64_t nz,
                          int32_t* __restrict__ coords) {
-    int64_t m = nx * ny * nz;
+    const int64_t m = nx * ny * nz;
     for (int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; c < m; c += int64_t(gridDim.x) * blockDim.x) {
-        int32_t r = rank[c];
+        const int32_t r = rank[c];
         if (r >= 0) {
-            int64_t k = c % nz, j = (c / nz) % ny, i = c / (ny * nz);
+            const IDX row = IDX(c) / IDX(nz), k = IDX(c) - row * IDX(nz);
+            const IDX i = row / IDX(ny), j = row - i * IDX(ny);
             coords[3 * int64_t(r)] = int32_t(i);
             coords[3 * int64_t(r) + 1] = int32_t(j);
             coords[3 * int64_t(r) + 2] = int32_t(k);
@@ -142,45 +132,68 @@ struct Grid {
     double dx;
 };
 
-__device__ inline int64_t wrap(int64_t x, int64_t s) { return ((x % s) + s) % s; }
-
-// Source cell of link i at node n: fills xyz, returns true when inside the grid.
-__device__ inline bool source_cell(const Grid& g, const int32_t* coords, int64_t n, int i, int64_t xyz[3]) {
-    const int cc[3] = {Lat::cx(i), Lat::cy(i), Lat::cz(i)};
-    bool inside = true;
-    for (int a = 0; a < 3; ++a) {
-        int64_t v = int64_t(coords[3 * n + a]) - cc[a];
-        if ((g.periodic >> a) & 1) v = wrap(v, g.dims[a]);
-        xyz[a] = v;
-        inside = inside && v >= 0 && v < g.dims[a];
-    }
-    return inside;
+// Coordinate v - c of one axis (c = -1, 0, 1), wrapped when the axis is periodic; -1 when it leaves the grid.
+template <class IDX>
+__device__ __forceinline__ IDX shifted(IDX v, int c, IDX dim, bool periodic) {
+    IDX x = v - IDX(c);
+    if (periodic) x = x < 0 ? x + dim : (x >= dim ? x - dim : x);
+    return x >= 0 && x < dim ? x : IDX(-1);
 }
 
-// Pass A: pull sources; count missing links per direction (len(miss) at lbm.py:294).
-__global__ void k_links_src(Grid g, const int32_t* __restrict__ coords, const int32_t* __restrict__ rank,
-                            int64_t n_fl, int32_t* __restrict__ nbr, float* __restrict__ q,
-                            int64_t* __restrict__ misses) {
+// Cell of node (x, y, z)'s pull source along link i, or -1 outside the grid.
+template <class IDX>
+__device__ __forceinline__ IDX source_cell(const Grid& g, IDX x, IDX y, IDX z, int cx, int cy, int cz, IDX out[3]) {
+    out[0] = shifted(x, cx, IDX(g.dims[0]), g.periodic & 1);
+    out[1] = shifted(y, cy, IDX(g.dims[1]), (g.periodic >> 1) & 1);
+    out[2] = shifted(z, cz, IDX(g.dims[2]), (g.periodic >> 2) & 1);
+    if (out[0] < 0 || out[1] < 0 || out[2] < 0) return IDX(-1);
+    return (out[0] * IDX(g.dims[1]) + out[1]) * IDX(g.dims[2]) + out[2];
+}
+
+// Pass A: pull sources; the missing links of each node as a mask of directions in miss_mask[3 n]; missing links per
+// direction (len(miss) at lbm.py:294). One thread per node finds all 27 sources, so its coordinates are read once and
+// the 27 reads of the rank grid hit the lines its neighbours read; bound by the 216 bytes a node writes. One thread
+// per link instead, with its 64-bit divisions, took 905 us on 839 k nodes.
+template <class IDX>
+__global__ void __launch_bounds__(256) k_links_src(Grid g, const int32_t* __restrict__ coords,
+                                                   const int32_t* __restrict__ rank, int64_t n_fl,
+                                                   int32_t* __restrict__ nbr, float* __restrict__ q,
+                                                   uint32_t* __restrict__ miss_mask, int64_t* __restrict__ misses) {
     __shared__ int miss_blk[Q];
     if (threadIdx.x < Q) miss_blk[threadIdx.x] = 0;
     __syncthreads();
-    int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-    if (t < n_fl * Q) {
-        int i = int(t / n_fl);
-        int64_t n = t - int64_t(i) * n_fl;
-        int64_t xyz[3];
-        int32_t src = CS_WALL;
-        if (source_cell(g, coords, n, i, xyz)) src = rank[(xyz[0] * g.dims[1] + xyz[1]) * g.dims[2] + xyz[2]];
-        if (src < 0) {
-            src = CS_WALL;
-            atomicAdd(&miss_blk[i], 1);
+    const int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    uint32_t mask = 0;
+    if (n < n_fl) {
+        const IDX x = coords[3 * n], y = coords[3 * n + 1], z = coords[3 * n + 2];
+        int32_t src[Q];
+#pragma unroll
+        for (int i = 0; i < Q; ++i) {
+            IDX cell[3];
+            const IDX c = source_cell<IDX>(g, x, y, z, Lat::cx(i), Lat::cy(i), Lat::cz(i), cell);
+            src[i] = c >= 0 ? __ldg(rank + c) : -1;
         }
-        nbr[t] = src;
-        q[t] = 0.5f;
+#pragma unroll
+        for (int i = 0; i < Q; ++i) {
+            if (src[i] < 0) mask |= 1u << i;
+            nbr[int64_t(i) * n_fl + n] = src[i] < 0 ? CS_WALL : src[i];
+            q[int64_t(i) * n_fl + n] = 0.5f;
+        }
+        miss_mask[3 * n] = mask;
+    }
+    if (__any_sync(0xffffffffu, mask != 0)) {
+        const int lane = threadIdx.x & 31;
+        int cnt = 0;
+#pragma unroll
+        for (int i = 0; i < Q; ++i) {
+            const unsigned b = __ballot_sync(0xffffffffu, (mask >> i) & 1u);
+            if (lane == i) cnt = __popc(b);
+        }
+        if (cnt) atomicAdd(&miss_blk[lane], cnt);
     }
     __syncthreads();
-    if (threadIdx.x < Q && miss_blk[threadIdx.x]) atomicAdd((unsigned long long*)&misses[threadIdx.x],
-                                                            (unsigned long long)miss_blk[threadIdx.x]);
+    if (threadIdx.x < Q && miss_blk[threadIdx.x])
+        atomicAdd((unsigned long long*)&misses[threadIdx.x], (unsigned long long)miss_blk[threadIdx.x]);
 }
 
 __device__ inline double row_dot(double x, double y, double z, const double* nv, bool single_row) {
@@ -188,93 +201,163 @@ __device__ inline double row_dot(double x, double y, double z, const double* nv,
     return __fma_rn(z, nv[2], __fma_rn(x, nv[0], __dmul_rn(y, nv[1])));
 }
 
-// Axial coordinate and distance from the opening's axis of point p (lbm.py:301-303).
-__device__ inline void axial_lateral(const double p[3], const double* c, const double* nv, bool single_row,
-                                     double* ax, double* lat) {
-    double r0 = __dsub_rn(p[0], c[0]), r1 = __dsub_rn(p[1], c[1]), r2 = __dsub_rn(p[2], c[2]);
-    double a = row_dot(r0, r1, r2, nv, single_row);
-    double v0 = __dsub_rn(r0, __dmul_rn(a, nv[0]));
-    double v1 = __dsub_rn(r1, __dmul_rn(a, nv[1]));
-    double v2 = __dsub_rn(r2, __dmul_rn(a, nv[2]));
-    *ax = a;
-    *lat = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(v0, v0), __dmul_rn(v1, v1)), __dmul_rn(v2, v2)));
+// Axial coordinate of point p along the opening, and what its distance from the axis needs (lbm.py:301-303).
+__device__ inline double axial(const double p[3], const double* c, const double* nv, bool single_row, double r[3]) {
+    for (int a = 0; a < 3; ++a) r[a] = __dsub_rn(p[a], c[a]);
+    return row_dot(r[0], r[1], r[2], nv, single_row);
 }
 
-// Pass B: classify missing links, wall q, link counts.
-__global__ void k_links_classify(Grid g, OpeningSet os, const float* __restrict__ phi,
-                                 const int32_t* __restrict__ coords, int64_t n_fl, const int64_t* __restrict__ misses,
-                                 int32_t* __restrict__ nbr, float* __restrict__ q, int64_t* __restrict__ counts,
-                                 int n_outlets) {
-    __shared__ unsigned long long cnt_blk[2 + MAX_OPENINGS];
-    for (int k = threadIdx.x; k < 2 + MAX_OPENINGS; k += blockDim.x) cnt_blk[k] = 0;
+__device__ inline double lateral(const double r[3], double ax, const double* nv) {
+    const double v0 = __dsub_rn(r[0], __dmul_rn(ax, nv[0]));
+    const double v1 = __dsub_rn(r[1], __dmul_rn(ax, nv[1]));
+    const double v2 = __dsub_rn(r[2], __dmul_rn(ax, nv[2]));
+    return __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(v0, v0), __dmul_rn(v1, v1)), __dmul_rn(v2, v2)));
+}
+
+constexpr int C_THREADS = 256;
+constexpr int C_NODES = 4 * C_THREADS;
+constexpr int C_LANES = 4;            // threads that share one boundary node's links
+
+// Pass B: classify missing links, wall q, link counts. A block compacts the nodes of its window that miss a link (about
+// one in ten) into shared memory and gives each of them four threads, so that whole warps work on links: testing every
+// link of every node took 309 us on 839 k nodes, most of it threads without work. It also clears the inlet profile,
+// whose first word per node brought the mask, and marks there the cells with an inlet link.
+template <class IDX>
+__global__ void __launch_bounds__(C_THREADS) k_links_classify(Grid g, OpeningSet os, const float* __restrict__ phi,
+                                                              const int32_t* __restrict__ coords, int64_t n_fl,
+                                                              const int64_t* __restrict__ misses,
+                                                              int32_t* __restrict__ nbr, float* __restrict__ q,
+                                                              float* __restrict__ uin, int64_t* __restrict__ counts,
+                                                              int n_outlets, int64_t* __restrict__ n_inlet_cells) {
+    __shared__ uint32_t s_mask[C_NODES];
+    __shared__ int16_t s_node[C_NODES];
+    __shared__ uint8_t s_inlet[C_NODES];
+    __shared__ int s_n, s_cells, s_cnt[2 + MAX_OPENINGS];
+    const int lane = threadIdx.x & 31;
+    const int64_t base = int64_t(blockIdx.x) * C_NODES;
+    if (threadIdx.x == 0) s_n = s_cells = 0;
+    for (int k = threadIdx.x; k < 2 + MAX_OPENINGS; k += C_THREADS) s_cnt[k] = 0;
     __syncthreads();
-    int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-    if (t < n_fl * Q && nbr[t] < 0) {
-        int i = int(t / n_fl);
-        int64_t n = t - int64_t(i) * n_fl;
-        int64_t xyz[3];
-        bool inside = source_cell(g, coords, n, i, xyz);
-        bool single = misses[i] == 1;
-        double p[3];
-        for (int a = 0; a < 3; ++a) p[a] = __dadd_rn(g.origin[a], __dmul_rn(double(xyz[a]), g.dx));
-        int32_t code = CS_WALL;
-        for (int o = 0; o < os.n; ++o) {
-            double ax, lat;
-            axial_lateral(p, os.c[o], os.nrm[o], single, &ax, &lat);
-            if (ax >= -1e-6 && lat < os.lim[o]) {
-                code = os.code[o];
-                break;
-            }
-        }
-        nbr[t] = code;
-        if (code == CS_WALL) {
-            int64_t m_here = (int64_t(coords[3 * n]) * g.dims[1] + coords[3 * n + 1]) * g.dims[2] + coords[3 * n + 2];
-            float px = phi[m_here];
-            float ps = __int_as_float(0x7fc00000);  // NaN outside the grid
-            if (inside) ps = phi[(xyz[0] * g.dims[1] + xyz[1]) * g.dims[2] + xyz[2]];
-            float qq = __fdiv_rn(-px, __fsub_rn(ps, px));
-            q[t] = isfinite(qq) ? fminf(fmaxf(qq, 0.001f), 1.0f) : 0.5f;
-            atomicAdd(&cnt_blk[0], 1ull);
-        } else if (code == CS_INLET) {
-            atomicAdd(&cnt_blk[1], 1ull);
-        } else {
-            atomicAdd(&cnt_blk[2 + (CS_OUTLET0 - code)], 1ull);
+#pragma unroll
+    for (int r = 0; r < C_NODES / C_THREADS; ++r) {
+        const int k = r * C_THREADS + threadIdx.x;
+        const uint32_t m = base + k < n_fl ? reinterpret_cast<const uint32_t*>(uin)[3 * (base + k)] : 0u;
+        const unsigned b = __ballot_sync(0xffffffffu, m != 0);
+        int at = 0;
+        if (lane == 0 && b) at = atomicAdd(&s_n, __popc(b));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(b & ((1u << lane) - 1u));
+        if (m) {
+            s_mask[at] = m;
+            s_node[at] = int16_t(k);
+            s_inlet[at] = 0;
         }
     }
     __syncthreads();
-    for (int k = threadIdx.x; k < 2 + n_outlets; k += blockDim.x)
-        if (cnt_blk[k]) atomicAdd((unsigned long long*)&counts[k], cnt_blk[k]);
+    const int64_t words = 3 * (min(n_fl - base, int64_t(C_NODES)));
+    for (int k = threadIdx.x; k < words; k += C_THREADS) uin[3 * base + k] = 0.0f;
+    const int entries = s_n;
+    int wall = 0, inlet = 0;
+    for (int w = threadIdx.x; w < entries * C_LANES; w += C_THREADS) {
+        const int e = w / C_LANES, part = w % C_LANES;
+        const int64_t n = base + s_node[e];
+        const IDX x = coords[3 * n], y = coords[3 * n + 1], z = coords[3 * n + 2];
+        const float px = phi[(x * IDX(g.dims[1]) + y) * IDX(g.dims[2]) + z];
+        int turn = 0;
+        for (uint32_t left = s_mask[e]; left; left &= left - 1, ++turn) {
+            if (turn % C_LANES != part) continue;
+            const int i = __ffs(left) - 1;
+            const int c3[3] = {k_c[0][i], k_c[1][i], k_c[2][i]};
+            IDX cell[3];
+            const IDX m = source_cell<IDX>(g, x, y, z, c3[0], c3[1], c3[2], cell);
+            // the source's position, outside the grid too (unwrapped there on no axis but the periodic ones)
+            const IDX at[3] = {x, y, z};
+            double p[3];
+            for (int a = 0; a < 3; ++a) {
+                const double v = cell[a] >= 0 ? double(cell[a]) : double(int64_t(at[a]) - c3[a]);
+                p[a] = __dadd_rn(g.origin[a], __dmul_rn(v, g.dx));
+            }
+            const bool single = misses[i] == 1;
+            int32_t code = CS_WALL;
+            for (int o = 0; o < os.n; ++o) {
+                double r[3];
+                const double ax = axial(p, os.c[o], os.nrm[o], single, r);
+                if (ax >= -1e-6 && lateral(r, ax, os.nrm[o]) < os.lim[o]) {
+                    code = os.code[o];
+                    break;
+                }
+            }
+            const int64_t t = int64_t(i) * n_fl + n;
+            if (code == CS_WALL) {
+                const float ps = m >= 0 ? phi[m] : __int_as_float(0x7fc00000);  // NaN outside the grid
+                const float qq = __fdiv_rn(-px, __fsub_rn(ps, px));
+                q[t] = isfinite(qq) ? fminf(fmaxf(qq, 0.001f), 1.0f) : 0.5f;
+                ++wall;
+            } else {
+                nbr[t] = code;
+                if (code == CS_INLET) {
+                    s_inlet[e] = 1;
+                    ++inlet;
+                } else {
+                    atomicAdd(&s_cnt[2 + (CS_OUTLET0 - code)], 1);
+                }
+            }
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        wall += __shfl_down_sync(0xffffffffu, wall, o);
+        inlet += __shfl_down_sync(0xffffffffu, inlet, o);
+    }
+    if (lane == 0) {
+        if (wall) atomicAdd(&s_cnt[0], wall);
+        if (inlet) atomicAdd(&s_cnt[1], inlet);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < entries; e += C_THREADS)
+        if (s_inlet[e]) {
+            reinterpret_cast<uint32_t*>(uin)[3 * (base + s_node[e])] = INLET_CELL;
+            atomicAdd(&s_cells, 1);
+        }
+    __syncthreads();
+    if (threadIdx.x == 0 && s_cells) atomicAdd((unsigned long long*)n_inlet_cells, (unsigned long long)s_cells);
+    for (int k = threadIdx.x; k < 2 + n_outlets; k += C_THREADS)
+        if (s_cnt[k]) atomicAdd((unsigned long long*)&counts[k], (unsigned long long)s_cnt[k]);
 }
 
-__global__ void k_inlet_cells(const int32_t* __restrict__ nbr, int64_t n_fl, int64_t* __restrict__ n_inlet_cells,
-                              float* __restrict__ uin) {
-    int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-    if (n >= n_fl) return;
-    bool any = false;
-    for (int i = 0; i < Q; ++i) any = any || nbr[int64_t(i) * n_fl + n] == CS_INLET;
-    uin[3 * n] = 0.0f;
-    uin[3 * n + 1] = 0.0f;
-    uin[3 * n + 2] = 0.0f;
-    if (any) atomicAdd((unsigned long long*)n_inlet_cells, 1ull);
-}
-
-__global__ void k_inlet_profile(Grid g, OpeningSet os, const int32_t* __restrict__ nbr,
-                                const int32_t* __restrict__ coords, int64_t n_fl,
+// Inlet profile of the marked cells, from the last inlet (lbm.py:322-328).
+__global__ void k_inlet_profile(Grid g, OpeningSet os, const int32_t* __restrict__ coords, int64_t n_fl,
                                 const int64_t* __restrict__ n_inlet_cells, float* __restrict__ uin) {
-    int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-    if (n >= n_fl || os.last_inlet < 0) return;
-    bool any = false;
-    for (int i = 0; i < Q; ++i) any = any || nbr[int64_t(i) * n_fl + n] == CS_INLET;
-    if (!any) return;
-    const int o = os.last_inlet;
-    double p[3];
-    for (int a = 0; a < 3; ++a) p[a] = __dadd_rn(g.origin[a], __dmul_rn(double(coords[3 * n + a]), g.dx));
-    double ax, lat;
-    axial_lateral(p, os.c[o], os.nrm[o], *n_inlet_cells == 1, &ax, &lat);
-    double r = __ddiv_rn(lat, os.radius[o]);
-    double prof = __dmul_rn(2.0, __dsub_rn(1.0, __dmul_rn(r, r)));
-    prof = prof < 0.0 ? 0.0 : prof;  // np.clip(., 0, None): NaN stays NaN
-    for (int a = 0; a < 3; ++a) uin[3 * n + a] = __double2float_rn(__dmul_rn(-prof, os.nrm[o][a]));
+    const int64_t n = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (n < n_fl && reinterpret_cast<const uint32_t*>(uin)[3 * n] == INLET_CELL) {
+        const int o = os.last_inlet;
+        double p[3], r[3];
+        for (int a = 0; a < 3; ++a) p[a] = __dadd_rn(g.origin[a], __dmul_rn(double(coords[3 * n + a]), g.dx));
+        const double ax = axial(p, os.c[o], os.nrm[o], *n_inlet_cells == 1, r);
+        const double rr = __ddiv_rn(lateral(r, ax, os.nrm[o]), os.radius[o]);
+        double prof = __dmul_rn(2.0, __dsub_rn(1.0, __dmul_rn(rr, rr)));
+        prof = prof < 0.0 ? 0.0 : prof;  // np.clip(., 0, None): NaN stays NaN
+        for (int a = 0; a < 3; ++a) uin[3 * n + a] = __double2float_rn(__dmul_rn(-prof, os.nrm[o][a]));
+    }
+}
+
+template <class IDX>
+int fill_tables(const Grid& g, const OpeningSet& os, const float* phi, const int32_t* rank, int64_t* misc, int64_t n_fluid,
+                int n_out, int32_t* nbr, float* q, float* uin, int32_t* coords, int64_t* counts, cudaStream_t st) {
+    const int64_t m = g.dims[0] * g.dims[1] * g.dims[2];
+    CS_CUDA(cudaMemsetAsync(misc + 1, 0, 28 * sizeof(int64_t), st));
+    k_coords<IDX><<<unsigned(std::min<int64_t>(ceil_div(m, 256), 148 * 64)), 256, 0, st>>>(rank, g.dims[0], g.dims[1],
+                                                                                         g.dims[2], coords);
+    CS_CHECK_LAUNCH("k_coords");
+    k_links_src<IDX><<<unsigned(ceil_div(n_fluid, 256)), 256, 0, st>>>(g, coords, rank, n_fluid, nbr, q,
+                                                                     reinterpret_cast<uint32_t*>(uin), misc + 1);
+    CS_CHECK_LAUNCH("k_links_src");
+    k_links_classify<IDX><<<unsigned(ceil_div(n_fluid, C_NODES)), C_THREADS, 0, st>>>(
+        g, os, phi, coords, n_fluid, misc + 1, nbr, q, uin, counts, n_out, misc + 28);
+    CS_CHECK_LAUNCH("k_links_classify");
+    if (os.last_inlet >= 0) {
+        k_inlet_profile<<<unsigned(ceil_div(n_fluid, 256)), 256, 0, st>>>(g, os, coords, n_fluid, misc + 28, uin);
+        CS_CHECK_LAUNCH("k_inlet_profile");
+    }
+    return CS_OK;
 }
 
 }  // namespace
@@ -353,24 +436,10 @@ extern "C" int cs_lattice_fill(const float* phi, int64_t nx, int64_t ny, int64_t
     char* s = static_cast<char*>(scratch);
     const int32_t* rank = reinterpret_cast<const int32_t*>(s + L.off_rank);
     int64_t* misc = reinterpret_cast<int64_t*>(s + L.off_misc);
-    Grid g{{nx, ny, nz}, periodic_mask & 7, {origin[0], origin[1], origin[2]}, dx};
-    int64_t m = nx * ny * nz;
-    k_coords<<<unsigned(std::min<int64_t>(ceil_div(m, 256), 148 * 64)), 256, 0, st>>>(rank, nx, ny, nz, coords);
-    CS_CHECK_LAUNCH("k_coords");
-    int64_t links = n_fluid * Q;
-    unsigned nb = unsigned(ceil_div(links, 256));
-    k_links_src<<<nb, 256, 0, st>>>(g, coords, rank, n_fluid, nbr, q, misc + 1);
-    CS_CHECK_LAUNCH("k_links_src");
-    k_links_classify<<<nb, 256, 0, st>>>(g, os, phi, coords, n_fluid, misc + 1, nbr, q, counts, n_out);
-    CS_CHECK_LAUNCH("k_links_classify");
-    unsigned nbn = unsigned(ceil_div(n_fluid, 256));
-    k_inlet_cells<<<nbn, 256, 0, st>>>(nbr, n_fluid, misc + 28, uin);
-    CS_CHECK_LAUNCH("k_inlet_cells");
-    if (os.last_inlet >= 0) {
-        k_inlet_profile<<<nbn, 256, 0, st>>>(g, os, nbr, coords, n_fluid, misc + 28, uin);
-        CS_CHECK_LAUNCH("k_inlet_profile");
-    }
-    return CS_OK;
+    const Grid g{{nx, ny, nz}, periodic_mask & 7, {origin[0], origin[1], origin[2]}, dx};
+    return nx * ny * nz < (int64_t(1) << 31)
+               ? fill_tables<int32_t>(g, os, phi, rank, misc, n_fluid, n_out, nbr, q, uin, coords, counts, st)
+               : fill_tables<int64_t>(g, os, phi, rank, misc, n_fluid, n_out, nbr, q, uin, coords, counts, st);
 }
 
 // ---- sponge (lbm.py:398-416) --------------------------------------------------------------------------------------

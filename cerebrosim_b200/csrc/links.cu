@@ -47,31 +47,8 @@ __global__ void k_ghost_count(const int32_t* __restrict__ nbr, int64_t n, int64_
 }
 
 // Exclusive scan of one direction's tile counts (block i); the total lands in part[i][tiles].
-__global__ void k_ghost_scan(int64_t* __restrict__ part, int64_t tiles) {
-    __shared__ int64_t s[1024];
-    int64_t* p = part + int64_t(blockIdx.x) * (tiles + 1);
-    const int64_t per = ceil_div(tiles, blockDim.x);
-    const int64_t lo = threadIdx.x * per, hi = min(lo + per, tiles);
-    int64_t sum = 0;
-    for (int64_t t = lo; t < hi; ++t) sum += p[t];
-    s[threadIdx.x] = sum;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int64_t run = 0;
-        for (int k = 0; k < (int)blockDim.x; ++k) {
-            const int64_t v = s[k];
-            s[k] = run;
-            run += v;
-        }
-        p[tiles] = run;
-    }
-    __syncthreads();
-    int64_t run = s[threadIdx.x];
-    for (int64_t t = lo; t < hi; ++t) {
-        const int64_t v = p[t];
-        p[t] = run;
-        run += v;
-    }
+__global__ void __launch_bounds__(1024) k_ghost_scan(int64_t* __restrict__ part, int64_t tiles) {
+    block_exclusive_scan(part + int64_t(blockIdx.x) * (tiles + 1), tiles);
 }
 
 __global__ void k_ghost_fill(const int32_t* __restrict__ nbr, const float* __restrict__ q, int64_t n, int n_out,
