@@ -215,13 +215,13 @@ __device__ inline double lateral(const double r[3], double ax, const double* nv)
 }
 
 constexpr int C_THREADS = 256;
-constexpr int C_NODES = 4 * C_THREADS;
-constexpr int C_LANES = 4;            // threads that share one boundary node's links
+constexpr int C_NODES = 512;
 
-// Pass B: classify missing links, wall q, link counts. A block compacts the nodes of its window that miss a link (about
-// one in ten) into shared memory and gives each of them four threads, so that whole warps work on links: testing every
-// link of every node took 309 us on 839 k nodes, most of it threads without work. It also clears the inlet profile,
-// whose first word per node brought the mask, and marks there the cells with an inlet link.
+// Pass B: classify missing links, wall q, link counts. A block lists the missing links of its window of nodes in shared
+// memory (one node in ten has any, then some seven) and gives each link a thread, so that whole warps work: a thread
+// per link of every node took 309 us on 839 k nodes, four threads per boundary node 154 (7.6 of 32 lanes at work), this
+// 41. It also clears the inlet profile, whose first word per node brought the mask, and marks there the cells with
+// an inlet link.
 template <class IDX>
 __global__ void __launch_bounds__(C_THREADS) k_links_classify(Grid g, OpeningSet os, const float* __restrict__ phi,
                                                               const int32_t* __restrict__ coords, int64_t n_fl,
@@ -229,77 +229,74 @@ __global__ void __launch_bounds__(C_THREADS) k_links_classify(Grid g, OpeningSet
                                                               int32_t* __restrict__ nbr, float* __restrict__ q,
                                                               float* __restrict__ uin, int64_t* __restrict__ counts,
                                                               int n_outlets, int64_t* __restrict__ n_inlet_cells) {
-    __shared__ uint32_t s_mask[C_NODES];
-    __shared__ int16_t s_node[C_NODES];
-    __shared__ uint8_t s_inlet[C_NODES];
+    __shared__ uint16_t s_link[C_NODES * Q];           // node in the window * 32 + direction
+    __shared__ uint8_t s_inlet[C_NODES], s_single[Q];
     __shared__ int s_n, s_cells, s_cnt[2 + MAX_OPENINGS];
     const int lane = threadIdx.x & 31;
     const int64_t base = int64_t(blockIdx.x) * C_NODES;
     if (threadIdx.x == 0) s_n = s_cells = 0;
+    if (threadIdx.x < Q) s_single[threadIdx.x] = misses[threadIdx.x] == 1;
     for (int k = threadIdx.x; k < 2 + MAX_OPENINGS; k += C_THREADS) s_cnt[k] = 0;
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < C_NODES / C_THREADS; ++r) {
         const int k = r * C_THREADS + threadIdx.x;
-        const uint32_t m = base + k < n_fl ? reinterpret_cast<const uint32_t*>(uin)[3 * (base + k)] : 0u;
-        const unsigned b = __ballot_sync(0xffffffffu, m != 0);
-        int at = 0;
-        if (lane == 0 && b) at = atomicAdd(&s_n, __popc(b));
-        at = __shfl_sync(0xffffffffu, at, 0) + __popc(b & ((1u << lane) - 1u));
-        if (m) {
-            s_mask[at] = m;
-            s_node[at] = int16_t(k);
-            s_inlet[at] = 0;
+        uint32_t m = base + k < n_fl ? reinterpret_cast<const uint32_t*>(uin)[3 * (base + k)] : 0u;
+        s_inlet[k] = 0;
+        if (!__any_sync(0xffffffffu, m != 0)) continue;
+        const int own = __popc(m);
+        int upto = own;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
         }
+        int at = 0;
+        if (lane == 31) at = atomicAdd(&s_n, upto);
+        at = __shfl_sync(0xffffffffu, at, 31) + upto - own;
+        for (; m; m &= m - 1) s_link[at++] = uint16_t(k * 32 + __ffs(m) - 1);
     }
     __syncthreads();
     const int64_t words = 3 * (min(n_fl - base, int64_t(C_NODES)));
     for (int k = threadIdx.x; k < words; k += C_THREADS) uin[3 * base + k] = 0.0f;
-    const int entries = s_n;
+    const int links = s_n;
     int wall = 0, inlet = 0;
-    for (int w = threadIdx.x; w < entries * C_LANES; w += C_THREADS) {
-        const int e = w / C_LANES, part = w % C_LANES;
-        const int64_t n = base + s_node[e];
-        const IDX x = coords[3 * n], y = coords[3 * n + 1], z = coords[3 * n + 2];
-        const float px = phi[(x * IDX(g.dims[1]) + y) * IDX(g.dims[2]) + z];
-        int turn = 0;
-        for (uint32_t left = s_mask[e]; left; left &= left - 1, ++turn) {
-            if (turn % C_LANES != part) continue;
-            const int i = __ffs(left) - 1;
-            const int c3[3] = {k_c[0][i], k_c[1][i], k_c[2][i]};
-            IDX cell[3];
-            const IDX m = source_cell<IDX>(g, x, y, z, c3[0], c3[1], c3[2], cell);
-            // the source's position, outside the grid too (unwrapped there on no axis but the periodic ones)
-            const IDX at[3] = {x, y, z};
-            double p[3];
-            for (int a = 0; a < 3; ++a) {
-                const double v = cell[a] >= 0 ? double(cell[a]) : double(int64_t(at[a]) - c3[a]);
-                p[a] = __dadd_rn(g.origin[a], __dmul_rn(v, g.dx));
+    for (int w = threadIdx.x; w < links; w += C_THREADS) {
+        const int e = s_link[w] >> 5, i = s_link[w] & 31;
+        const int64_t n = base + e;
+        const IDX at[3] = {IDX(coords[3 * n]), IDX(coords[3 * n + 1]), IDX(coords[3 * n + 2])};
+        const int c3[3] = {k_c[0][i], k_c[1][i], k_c[2][i]};
+        IDX cell[3];
+        const IDX m = source_cell<IDX>(g, at[0], at[1], at[2], c3[0], c3[1], c3[2], cell);
+        const float px = phi[(at[0] * IDX(g.dims[1]) + at[1]) * IDX(g.dims[2]) + at[2]];
+        const float ps = m >= 0 ? phi[m] : __int_as_float(0x7fc00000);       // NaN outside the grid
+        // the source's position, wrapped on the periodic axes only
+        double p[3];
+        for (int a = 0; a < 3; ++a) {
+            const IDX v = cell[a] >= 0 ? cell[a] : at[a] - IDX(c3[a]);
+            p[a] = __dadd_rn(g.origin[a], __dmul_rn(double(v), g.dx));
+        }
+        const bool single = s_single[i] != 0;
+        int32_t code = CS_WALL;
+        for (int o = 0; o < os.n; ++o) {
+            double r[3];
+            const double ax = axial(p, os.c[o], os.nrm[o], single, r);
+            if (ax >= -1e-6 && lateral(r, ax, os.nrm[o]) < os.lim[o]) {
+                code = os.code[o];
+                break;
             }
-            const bool single = misses[i] == 1;
-            int32_t code = CS_WALL;
-            for (int o = 0; o < os.n; ++o) {
-                double r[3];
-                const double ax = axial(p, os.c[o], os.nrm[o], single, r);
-                if (ax >= -1e-6 && lateral(r, ax, os.nrm[o]) < os.lim[o]) {
-                    code = os.code[o];
-                    break;
-                }
-            }
-            const int64_t t = int64_t(i) * n_fl + n;
-            if (code == CS_WALL) {
-                const float ps = m >= 0 ? phi[m] : __int_as_float(0x7fc00000);  // NaN outside the grid
-                const float qq = __fdiv_rn(-px, __fsub_rn(ps, px));
-                q[t] = isfinite(qq) ? fminf(fmaxf(qq, 0.001f), 1.0f) : 0.5f;
-                ++wall;
+        }
+        const int64_t t = int64_t(i) * n_fl + n;
+        if (code == CS_WALL) {
+            const float qq = __fdiv_rn(-px, __fsub_rn(ps, px));
+            q[t] = isfinite(qq) ? fminf(fmaxf(qq, 0.001f), 1.0f) : 0.5f;
+            ++wall;
+        } else {
+            nbr[t] = code;
+            if (code == CS_INLET) {
+                s_inlet[e] = 1;
+                ++inlet;
             } else {
-                nbr[t] = code;
-                if (code == CS_INLET) {
-                    s_inlet[e] = 1;
-                    ++inlet;
-                } else {
-                    atomicAdd(&s_cnt[2 + (CS_OUTLET0 - code)], 1);
-                }
+                atomicAdd(&s_cnt[2 + (CS_OUTLET0 - code)], 1);
             }
         }
     }
@@ -312,9 +309,9 @@ __global__ void __launch_bounds__(C_THREADS) k_links_classify(Grid g, OpeningSet
         if (inlet) atomicAdd(&s_cnt[1], inlet);
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < entries; e += C_THREADS)
+    for (int e = threadIdx.x; e < C_NODES; e += C_THREADS)
         if (s_inlet[e]) {
-            reinterpret_cast<uint32_t*>(uin)[3 * (base + s_node[e])] = INLET_CELL;
+            reinterpret_cast<uint32_t*>(uin)[3 * (base + e)] = INLET_CELL;
             atomicAdd(&s_cells, 1);
         }
     __syncthreads();
