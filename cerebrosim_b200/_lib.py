@@ -47,7 +47,8 @@ class StepDesc(ctypes.Structure):
                 ("q_part", ctypes.c_void_p), ("fb_list", ctypes.c_void_p), ("n_fb", ctypes.c_int32),
                 ("q_last", ctypes.c_void_p), ("p_out64", ctypes.c_void_p),
                 ("r_out", ctypes.c_void_p), ("pref", ctypes.c_double), ("alpha", ctypes.c_double),
-                ("gblock", ctypes.c_int32 * 28), ("beat_acc", ctypes.c_void_p)]
+                ("gblock", ctypes.c_int32 * 28), ("beat_acc", ctypes.c_void_p), ("drive2", ctypes.c_void_p), ("fstride", ctypes.c_int64),
+                ("vstride", ctypes.c_int64)]
 
 
 class BatchDesc(ctypes.Structure):

@@ -1,17 +1,16 @@
 // Sparse D3Q27 step on the GPU: lbm.k_clock + lbm.k_step (lbm.py:90-257) and, for the artery solver,
 // simulate.k_flux + simulate.k_bc (simulate.py:65-82).
 //
-// One step = two or three kernels on one stream:
-//  1. k_boundary — the wall / inlet / outlet link list (lbm.py:163-181) and the clock (lbm.py:94-102). One thread
-//     per ghost slot (a boundary link of one direction); it evaluates what the reference's pull produces for that
-//     link — Bouzidi interpolation (q < 0.5 with the second node, q >= 0.5 with the node's own population),
-//     half-way bounce-back, the velocity inlet with the drive, the pressure outlet with p_out and the previous
-//     velocity — and stores it in the ghost slot f_in[i * npad + n + g] of the step's input buffer. Its first
-//     thread evaluates drive(tick[a]) into *drive and advances tick[1 - a] = tick[a] + 1; nothing else in the step
-//     reads tick[1 - a], and the bulk kernel reads the drive from memory instead of recomputing it.
+// One step = two or three kernels on one stream, each launched programmatically so that its blocks start under the last
+// one's (all with one division of the SM's memory: set_carveout), after a one-warp k_clock once per call:
+//  1. k_boundary — the wall / inlet / outlet link list (lbm.py:163-181). One thread per ghost slot (a boundary link of
+//     one direction); it evaluates what the reference's pull produces for that link — Bouzidi interpolation (q < 0.5
+//     with the second node, q >= 0.5 with the node's own population), half-way bounce-back, the velocity inlet with the
+//     drive, the pressure outlet with p_out and the previous velocity — and stores it in the ghost slot
+//     f_in[i * fstride + n + g] of the step's input buffer.
 //  2. k_bulk (k_bulk_dense: the regularised step without body force in blocks of <= 128 threads, 9 per SM) — one
 //     thread per fluid node, C-ordered nodes, link-major populations (the reference's SoA layout).
-//     Every link is a plain pull f_in[i * npad + links[i * n + node]] (a fluid source or a ghost slot), so the 27
+//     Every link is a plain pull f_in[i * fstride + links[i * n + node]] (a fluid source or a ghost slot), so the 27
 //     loads carry no branch and issue back to back; for each link the warp's 32 sources are mostly consecutive,
 //     so each load and store moves whole 128-byte lines. Links come in pairs (i, opp(i)) with c_opp = -c_i: the
 //     pull accumulates dr, j and Pi = sum c c^T f from each pair's sum and difference, and the collision output is
@@ -21,7 +20,9 @@
 //     (lbm.py:192-204) from the six axis neighbours' previous velocity (a ghost slot gives the wall's q or marks an
 //     opening); cells with an inlet link (om < 0) get the inlet equilibrium (lbm.py:205-216); TRT (lbm.py:241-255)
 //     keeps the populations.
-//  3. k_bc (only with the resistance coupling) — one block: p_out[0] = drive, p_out[k] relaxed towards R_k Q_k -
+//     Its first block is the clock (lbm.py:94-102): it stores this step's drive, advances tick[1 - a] = tick[a] + 1 and
+//     evaluates the next step's drive.
+//  3. k_bc (only with the resistance coupling) — one block, launched programmatically too: p_out[0] = drive, p_out[k] relaxed towards R_k Q_k -
 //     pref in FP64, Qlast = Q, Q = 0 (simulate.py:76-82). The slab flux Q_k = sum u . w itself is reduced in the
 //     bulk kernel in FP64 by the blocks that hold flux cells (simulate.py:65-69).
 #include <cuda_bf16.h>
@@ -29,6 +30,7 @@
 
 #include "cs_common.cuh"
 
+#include <utility>
 #include <vector>
 
 namespace cs {
@@ -44,8 +46,18 @@ __constant__ int k_cx[Q] = {0, 1, -1, 0, 0, 0, 0, 1, -1, 1, -1, 1, -1, 1, -1, 0,
 __constant__ int k_cy[Q] = {0, 0, 0, 1, -1, 0, 0, 1, -1, -1, 1, 0, 0, 0, 0, 1, -1, 1, -1, 1, -1, 1, -1, -1, 1, 1, -1};
 __constant__ int k_cz[Q] = {0, 0, 0, 0, 0, 1, -1, 0, 0, 0, 0, 1, -1, -1, 1, 1, -1, -1, 1, 1, -1, -1, 1, 1, -1, 1, -1};
 
+__device__ __forceinline__ float weight_rt(int i) {
+    return i == 0 ? 8.0f / 27.0f : (i < 7 ? 2.0f / 27.0f : (i < 19 ? 1.0f / 54.0f : 1.0f / 216.0f));
+}
+
+// 1024 / w_i of the 16-bit formats for a link known at run time, without a division at run time.
+__device__ __forceinline__ float scale_rt(int i) {
+    constexpr float s0 = 1024.0f / wgt(0), s1 = 1024.0f / wgt(1), s7 = 1024.0f / wgt(7), s19 = 1024.0f / wgt(19);
+    return i == 0 ? s0 : (i < 7 ? s1 : (i < 19 ? s7 : s19));
+}
+
 // ---- population storage -----------------------------------------------------------------------------------------
-// 32-bit element offsets: 27 * npad < 2^31 is checked on the host.
+// 32-bit element offsets: 27 * fstride < 2^31 is checked on the host.
 template <int ST> struct Pop;
 
 template <> struct Pop<CS_STORE_F32> {
@@ -53,6 +65,7 @@ template <> struct Pop<CS_STORE_F32> {
         return __ldg(static_cast<const float*>(b) + idx);
     }
     static __device__ __forceinline__ void st(void* b, uint32_t idx, float, float v) { static_cast<float*>(b)[idx] = v; }
+    static __device__ __forceinline__ void st_link(void* b, uint32_t idx, int, float v) { static_cast<float*>(b)[idx] = v; }
 };
 
 // 16-bit formats store (f - w_i) * 1024 / w_i: all links share one range, well inside FP16's normal numbers, so the
@@ -68,6 +81,10 @@ template <> struct Pop<CS_STORE_F16> {
     static __device__ __forceinline__ void st_scaled(void* b, uint32_t idx, float g) {
         static_cast<__half*>(b)[idx] = __float2half_rn(g);
     }
+    // a value of link i, known at run time
+    static __device__ __forceinline__ void st_link(void* b, uint32_t idx, int i, float v) {
+        static_cast<__half*>(b)[idx] = __float2half_rn(v * scale_rt(i));
+    }
 };
 
 template <> struct Pop<CS_STORE_BF16> {
@@ -79,6 +96,10 @@ template <> struct Pop<CS_STORE_BF16> {
     }
     static __device__ __forceinline__ void st_scaled(void* b, uint32_t idx, float g) {
         static_cast<__nv_bfloat16*>(b)[idx] = __float2bfloat16_rn(g);
+    }
+    // a value of link i, known at run time
+    static __device__ __forceinline__ void st_link(void* b, uint32_t idx, int i, float v) {
+        static_cast<__nv_bfloat16*>(b)[idx] = __float2bfloat16_rn(v * scale_rt(i));
     }
 };
 
@@ -93,16 +114,35 @@ __device__ __forceinline__ float drive_value(const cs_step_desc& d, int t) {
     return v;
 }
 
+// The same by a whole warp, each lane one term's sine or cosine: a thread alone waits for its coefficients from memory one
+// harmonic after the other (4 us for three).
+__device__ __forceinline__ float drive_value_warp(const cs_step_desc& d, int t) {
+    const int lane = threadIdx.x & 31;
+    const float ph = 2.0f * PI_F * float(t % d.period) / float(d.period);
+    float v = d.coef[0];
+    for (int k0 = 1; k0 <= d.nh; k0 += 16) {
+        const int k = k0 + (lane >> 1);
+        float c = 0.0f, f = 0.0f;
+        if (k <= d.nh) {
+            c = d.coef[2 * k - 1 + (lane & 1)];
+            f = lane & 1 ? sinf(float(k) * ph) : cosf(float(k) * ph);
+        }
+        for (int j = 0; j < 16 && k0 + j <= d.nh; ++j) {
+            const float cc = __shfl_sync(0xffffffffu, c, 2 * j), cs_ = __shfl_sync(0xffffffffu, c, 2 * j + 1);
+            const float fc = __shfl_sync(0xffffffffu, f, 2 * j), fs = __shfl_sync(0xffffffffu, f, 2 * j + 1);
+            v += __fmaf_rn(cs_, fs, cc * fc);       // as the compiler contracts the sum in one thread
+        }
+    }
+    if (t < d.ramp) v *= 0.5f - 0.5f * cosf(PI_F * float(t) / float(d.ramp));
+    return v;
+}
+
 // Programmatic dependent launch (sm_90+): a kernel launched with the programmatic-serialization attribute may start
 // while the previous kernel of the stream is still running; it reads only static tables until
 // grid_dependency_wait(), which returns once that kernel has completed and its writes are visible. A kernel calls
 // launch_dependents() once the next kernel may be scheduled beside it. Both are no-ops for an ordinary launch.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" :::); }
-
-__device__ __forceinline__ float weight_rt(int i) {
-    return i == 0 ? 8.0f / 27.0f : (i < 7 ? 2.0f / 27.0f : (i < 19 ? 1.0f / 54.0f : 1.0f / 216.0f));
-}
 
 // Non-uniform central difference (lbm.py:105-126) of one velocity component: gm / gp are the values loaded through
 // the links that pull from x - e_a (sm) and x + e_a (sp) — the neighbour's previous velocity component for a fluid
@@ -129,7 +169,7 @@ __device__ __forceinline__ float ddx_g(int32_t sm, int32_t sp, float gm, float g
 // Address of what the difference along link k (1..6) reads for velocity component c: the neighbour's component, or
 // the ghost slot's q.
 __device__ __forceinline__ const float* grad_src(const cs_step_desc& d, const float* vin, int k, int c, int32_t s) {
-    return s < d.n ? vin + int64_t(c) * d.n + s : d.gq + int64_t(k) * d.gmax + (s - d.n);
+    return s < d.n ? vin + int64_t(c) * d.vstride + s : d.gq + int64_t(k) * d.gmax + (s - d.n);
 }
 
 // Third-order equilibrium term of link I (lbm.py:129-137) from the velocity monomials; odd in c.
@@ -340,85 +380,85 @@ __device__ __forceinline__ void store_regularised(void* fout, uint32_t NP, int32
 }
 
 // ---- 1. boundary-link kernel and clock ----------------------------------------------------------------------------
-// Block (bx, by) of a lattice's boundary-link grid: by = direction, bx = chunk of its ghost slots.
+// The clock. A step reads its drive, drive2[a], from memory: evaluating it (coefficients from memory, a sine and a
+// cosine per harmonic) took about 4 us on the step's critical path, in the boundary kernel that everything waits for.
+// The bulk kernel of the step before evaluates it beside its nodes, k_clock before the first step of a call.
+__device__ __forceinline__ void advance_clock(const cs_step_desc& d, const int a) {
+    const int t = d.tick[a];
+    const float next = drive_value_warp(d, t + 1);
+    if ((threadIdx.x & 31) == 0) {
+        *d.drive = d.drive2[a];
+        d.drive2[1 - a] = next;
+        d.tick[1 - a] = t + 1;
+    }
+}
+
+__device__ __forceinline__ void first_clock(const cs_step_desc& d, const int a) {
+    const float v = drive_value_warp(d, d.tick[a]);
+    if (threadIdx.x == 0) d.drive2[a] = v;
+}
+
+__global__ void __launch_bounds__(32) k_clock(const cs_step_desc d, const int a) { first_clock(d, a); }
+
+// Without nodes there is no bulk kernel to advance the clock.
+__global__ void __launch_bounds__(32) k_clock_only(const cs_step_desc d, const int a) { advance_clock(d, a); }
+
+// Block (bx, by) of a lattice's boundary-link grid: by = direction, bx = chunk of its ghost slots. Pure latency: the
+// slot's table words (static, read before the previous kernel has ended), its two populations, the ghost's write. Both
+// populations are addressed without a branch, so their loads are in flight together.
 template <int ST>
-__device__ __forceinline__ void boundary_body(const cs_step_desc& d, const int a, const int bx, const int by,
-                                              const bool clock) {
-    // the ghost table is static: read it before waiting for the previous kernel of the stream
+__device__ __forceinline__ void boundary_body(const cs_step_desc& d, const int a, const int bx, const int by) {
     const int i = by;
-    const int64_t g = int64_t(bx) * B_THREADS + threadIdx.x;
-    const int64_t slot = int64_t(i) * d.gmax + g;
+    const int32_t g = bx * B_THREADS + int(threadIdx.x);
+    const uint32_t slot = uint32_t(i) * uint32_t(d.gmax) + uint32_t(g);       // < 27 npad < 2^31
     const bool live = g < d.gmax;
     const int32_t node = live ? __ldg(d.gnode + slot) : -1;
     const int32_t info = live ? __ldg(d.ginfo + slot) : 0;
-    const float qslot = live ? __ldg(d.gq + slot) : 0.0f;
-    grid_dependency_wait();
-    // issue the slot's loads first: the clock below (one thread, then a barrier) overlaps their latency
+    const float q = live ? __ldg(d.gq + slot) : 0.0f;
     const int io = Lat::opp(i);
-    const float w = weight_rt(i), wo = weight_rt(io);
-    const uint32_t NP = uint32_t(d.npad);
-    const void* fin = d.f[a];
-    const bool live_node = node >= 0;
-    const uint32_t nn = live_node ? uint32_t(node) : 0u;
-    const bool is_wall = info >= CS_WALL, is_inlet = info == CS_INLET;
-    float fo = 0.0f, f2 = 0.0f, e0 = 0.0f, e1 = 0.0f, e2 = 0.0f, pk = 0.0f;
-    if (live_node) {
-        fo = Pop<ST>::ld(fin, uint32_t(io) * NP + nn, wo);
-        if (is_wall) {
-            if (d.bouzidi) {
-                if (qslot < 0.5f) {
-                    if (info >= 0) f2 = Pop<ST>::ld(fin, uint32_t(io) * NP + uint32_t(info), wo);
-                } else {
-                    f2 = Pop<ST>::ld(fin, uint32_t(i) * NP + nn, w);
-                }
-            }
-        } else if (is_inlet) {
-            const float* u = d.uin + 3 * int64_t(node);
-            e0 = __ldg(u);
-            e1 = __ldg(u + 1);
-            e2 = __ldg(u + 2);
-        } else {
-            const float* vin = d.vel[a];
-            e0 = __ldg(vin + node);
-            e1 = __ldg(vin + d.n + node);
-            e2 = __ldg(vin + 2 * d.n + node);
-            pk = __ldg(d.p_out + (CS_OUTLET0 - info));
-        }
-    }
-    // the clock: the first thread of the grid publishes this step's drive and advances the tick; an inlet link
-    // evaluates the drive itself (no block waits for one thread's evaluation)
-    if (threadIdx.x == 0 && clock) {
-        const int t = d.tick[a];
-        *d.drive = drive_value(d, t);
-        d.tick[1 - a] = t + 1;
-    }
+    const uint32_t NP = uint32_t(d.fstride), own = uint32_t(io) * NP + uint32_t(node);
+    // Bouzidi's second population: the wall's second node (q < 0.5) or the node's own along i
+    const bool second = info >= 0 && q < 0.5f;
+    const uint32_t other = second ? uint32_t(io) * NP + uint32_t(info) : uint32_t(i) * NP + uint32_t(node);
+    const float w = weight_rt(i);                                             // the opposite's weight too
+    grid_dependency_wait();
     launch_dependents();                                    // the bulk kernel may start its static loads
-    if (!live_node) return;                                 // padding slot of a direction with fewer links
-    const float cx = float(k_cx[i]), cy = float(k_cy[i]), cz = float(k_cz[i]);
+    if (node < 0) return;                                   // padding slot of a direction with fewer links
+    const void* fin = d.f[a];
+    const float fo = Pop<ST>::ld(fin, own, w);
     float v;
-    if (is_wall) {
+    if (info >= CS_WALL) {
         // lbm.py:163-173: interpolated bounce-back, or half-way bounce-back without Bouzidi
+        const float f2 = Pop<ST>::ld(fin, other, w);
         v = fo;
         if (d.bouzidi) {
-            const float q = qslot;
             if (q < 0.5f) {
-                if (info >= 0) v = 2.0f * q * fo + (1.0f - 2.0f * q) * f2;
+                if (second) v = 2.0f * q * fo + (1.0f - 2.0f * q) * f2;
             } else {
                 v = fo / (2.0f * q) + (2.0f * q - 1.0f) / (2.0f * q) * f2;
             }
         }
-    } else if (is_inlet) {
-        // lbm.py:174-177: bounce-back with the prescribed velocity
-        const float dv = drive_value(d, d.tick[a]);
-        const float cu = cx * (e0 * dv) + cy * (e1 * dv) + cz * (e2 * dv);
-        v = fo + 6.0f * w * cu;
     } else {
-        // lbm.py:178-181: anti-bounce-back with the outlet's pressure and the previous velocity
-        const float cu = cx * e0 + cy * e1 + cz * e2;
-        const float usq = e0 * e0 + e1 * e1 + e2 * e2;
-        v = -fo + 2.0f * w * (3.0f * pk + 4.5f * cu * cu - 1.5f * usq);
+        const float cx = float(k_cx[i]), cy = float(k_cy[i]), cz = float(k_cz[i]);
+        if (info == CS_INLET) {
+            // lbm.py:174-177: bounce-back with the prescribed velocity
+            const float* u = d.uin + 3 * int64_t(node);
+            const float dv = d.drive2[a];
+            const float cu = cx * (__ldg(u) * dv) + cy * (__ldg(u + 1) * dv) + cz * (__ldg(u + 2) * dv);
+            v = fo + 6.0f * w * cu;
+        } else {
+            // lbm.py:178-181: anti-bounce-back with the outlet's pressure and the previous velocity
+            const float* vin = d.vel[a];
+            const float e0 = __ldg(vin + node), e1 = __ldg(vin + d.vstride + node), e2 = __ldg(vin + 2 * d.vstride + node);
+            const float pk = __ldg(d.p_out + (CS_OUTLET0 - info));
+            const float cu = cx * e0 + cy * e1 + cz * e2;
+            // (rounded as spelled out, so that the result does not hang on the compiler's choice of what to fuse)
+            const float usq = __fmaf_rn(e2, e2, __fmaf_rn(e0, e0, e1 * e1));
+            const float eq = __fmaf_rn(-1.5f, usq, __fmaf_rn(4.5f * cu, cu, 3.0f * pk));
+            v = __fmaf_rn(2.0f * w, eq, -fo);
+        }
     }
-    Pop<ST>::st(d.f[a], uint32_t(i) * NP + uint32_t(d.n + g), w, v);
+    Pop<ST>::st_link(d.f[a], uint32_t(i) * NP + uint32_t(d.n) + uint32_t(g), i, v);
 }
 
 // Direction of block b of the unpadded boundary grid: the largest i with gblock[i] <= b.
@@ -432,15 +472,15 @@ __device__ __forceinline__ int grid_direction(const int32_t* gblock, int b) {
 }
 
 // Work item `item` of a lattice's boundary-link grid: a 256-slot chunk of one direction (unpadded grid when gblock
-// is set, else ceil(gmax / 256) chunks per direction); item 0 advances the clock.
+// is set, else ceil(gmax / 256) chunks per direction).
 template <int ST>
 __device__ __forceinline__ void boundary_item(const cs_step_desc& d, const int a, const int item) {
     if (d.gblock[Q] > 0) {
         const int i = grid_direction(d.gblock, item);
-        boundary_body<ST>(d, a, item - d.gblock[i], i, item == 0);
+        boundary_body<ST>(d, a, item - d.gblock[i], i);
     } else {
         const int nbx = int(max(int64_t(1), ceil_div(d.gmax, B_THREADS)));
-        boundary_body<ST>(d, a, item % nbx, item / nbx, item == 0);
+        boundary_body<ST>(d, a, item % nbx, item / nbx);
     }
 }
 
@@ -475,8 +515,8 @@ __device__ __forceinline__ void store_pairs(void* fout, uint32_t NP, int32_t n, 
 template <int ST, int MODEL, bool GAL, bool FORCE>
 __device__ __forceinline__ void node_update(const cs_step_desc& d, int a, int32_t n, float& ux_o, float& uy_o,
                                             float& uz_o) {
-    const int32_t N = int32_t(d.n);
-    const uint32_t NP = uint32_t(d.npad);
+    const int32_t N = int32_t(d.n), NV = int32_t(d.vstride);
+    const uint32_t NP = uint32_t(d.fstride);
     const void* fin = d.f[a];
     void* fout = d.f[1 - a];
     const float* vin = d.vel[a];
@@ -502,8 +542,8 @@ __device__ __forceinline__ void node_update(const cs_step_desc& d, int a, int32_
     }
     const float om_signed = __ldg(d.om + n);
     grid_dependency_wait();
-    const float dv = __ldg(d.drive);
-    const float upx = __ldg(vin + n), upy = __ldg(vin + N + n), upz = __ldg(vin + 2 * N + n);
+    const float dv = __ldg(d.drive2 + a);
+    const float upx = __ldg(vin + n), upy = __ldg(vin + NV + n), upz = __ldg(vin + 2 * NV + n);
 
     // six loads for the Galilean differences, issued with the pull
     float g[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -552,8 +592,8 @@ __device__ __forceinline__ void node_update(const cs_step_desc& d, int a, int32_
             o = 3.0f * cu + t3 * cu3.template h3<I>();
         });
         vout[n] = tx;
-        vout[N + n] = ty;
-        vout[2 * N + n] = tz;
+        vout[NV + n] = ty;
+        vout[2 * NV + n] = tz;
         d.rho[n] = dr;
         ux_o = tx;
         uy_o = ty;
@@ -632,8 +672,8 @@ __device__ __forceinline__ void node_update(const cs_step_desc& d, int a, int32_
                 Pop<ST>::st(fout, uint32_t(O) * NP + uint32_t(n), w, feq_o + k_ne * fneq_o + k_src * src_o);
             });
             vout[n] = ux;
-            vout[N + n] = uy;
-            vout[2 * N + n] = uz;
+            vout[NV + n] = uy;
+            vout[2 * NV + n] = uz;
             d.rho[n] = dr;
             ux_o = ux;
             uy_o = uy;
@@ -672,8 +712,8 @@ __device__ __forceinline__ void node_update(const cs_step_desc& d, int a, int32_
         });
     }
     vout[n] = ux;
-    vout[N + n] = uy;
-    vout[2 * N + n] = uz;
+    vout[NV + n] = uy;
+    vout[2 * NV + n] = uz;
     d.rho[n] = dr;
     ux_o = ux;
     uy_o = uy;
@@ -681,60 +721,83 @@ __device__ __forceinline__ void node_update(const cs_step_desc& d, int a, int32_
 }
 
 // Block bx of a lattice's bulk grid (nodes bx * blockDim .. + blockDim - 1). Called by every thread of the block.
-template <int ST, int MODEL, bool GAL, bool FORCE>
-__device__ __forceinline__ void bulk_body(const cs_step_desc& d, const int a, const int bx) {
-    __shared__ float s_u[3][MAX_BLOCK];
+// OPEN: the lattice may have open ends (n_open > 0); compiled apart for the kernels that lose by carrying their
+// reduction. clock: this block also advances the clock.
+template <int ST, int MODEL, bool GAL, bool FORCE, bool OPEN>
+__device__ __forceinline__ void bulk_body(const cs_step_desc& d, const int a, const int bx, const bool clock) {
     const int32_t n0 = int32_t(bx) * int32_t(blockDim.x);
     const int32_t n = n0 + int32_t(threadIdx.x);
+    // read after the update: bring the line in meanwhile, at the cost of no register
+    if (OPEN && d.n_open > 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(d.flux_block + bx));
     float ux = 0.f, uy = 0.f, uz = 0.f;
     if (n < d.n) node_update<ST, MODEL, GAL, FORCE>(d, a, n, ux, uy, uz);
     grid_dependency_wait();      // (threads without a node) the flux accumulators were reset by the last step
     launch_dependents();
+    if (clock && threadIdx.x < 32) advance_clock(d, a);
 
-    if (d.n_open > 0) {
+    if (OPEN && d.n_open > 0) {
         // slab flux Q_k = sum u . w over this block's flux entries (simulate.py:65-69), FP64, in a fixed order: each
-        // thread sums its entries, warps reduce by shuffles, warp 0 adds the warps in order; the block's partial
-        // sums go to its own row of q_part, which k_bc adds up in a fixed order too (no atomics: bit-reproducible)
+        // thread sums its entries, warps reduce by shuffles, the warps' sums are added in order; the block's partial
+        // sums go to its own row of q_part, which k_bc adds up in a fixed order too (no atomics: bit-reproducible).
+        // In an order along the vessel nearly every block holds a few entries (7 of 128 nodes on a 190 k-node
+        // artery), so only the warps and open ends that have any take part.
         const int e0 = __ldg(d.flux_block + bx), e1 = __ldg(d.flux_block + bx + 1);
         if (e1 > e0) {
+            __shared__ float s_u[3][MAX_BLOCK];
             s_u[0][threadIdx.x] = ux;
             s_u[1][threadIdx.x] = uy;
             s_u[2][threadIdx.x] = uz;
             __syncthreads();
-            double acc[MAX_OPEN];
-#pragma unroll
-            for (int k = 0; k < MAX_OPEN; ++k) acc[k] = 0.0;
-            for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-                const int loc = __ldg(d.flux_idx + e) - n0;
-                if (loc < 0 || loc >= int(blockDim.x)) continue;  // partition built for another block size
-                const float* w = d.flux_w + 3 * int64_t(e);
-                const double v = double(s_u[0][loc]) * double(__ldg(w)) + double(s_u[1][loc]) * double(__ldg(w + 1)) +
-                                 double(s_u[2][loc]) * double(__ldg(w + 2));
-                const int slot = __ldg(d.flux_slot + e);
-#pragma unroll
-                for (int k = 0; k < MAX_OPEN; ++k) acc[k] += slot == k ? v : 0.0;
-            }
             __shared__ double s_w[MAX_BLOCK / 32][MAX_OPEN];
             const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+            const int busy = min(int(blockDim.x) / 32, (e1 - e0 + 31) / 32);
+            if (warp < busy) {
+                double acc[MAX_OPEN];
 #pragma unroll
-            for (int k = 0; k < MAX_OPEN; ++k) {
-                double x = acc[k];
-                for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-                if (lane == 0) s_w[warp][k] = x;
+                for (int k = 0; k < MAX_OPEN; ++k) acc[k] = 0.0;
+                for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
+                    const int loc = __ldg(d.flux_idx + e) - n0;
+                    if (loc < 0 || loc >= int(blockDim.x)) continue;  // partition built for another block size
+                    const float* w = d.flux_w + 3 * int64_t(e);
+                    const double v = double(s_u[0][loc]) * double(__ldg(w)) + double(s_u[1][loc]) * double(__ldg(w + 1)) +
+                                     double(s_u[2][loc]) * double(__ldg(w + 2));
+                    const int slot = __ldg(d.flux_slot + e);
+#pragma unroll
+                    for (int k = 0; k < MAX_OPEN; ++k) acc[k] += slot == k ? v : 0.0;
+                }
+#pragma unroll
+                for (int k = 0; k < MAX_OPEN; ++k) {
+                    if (k >= d.n_open) break;
+                    double x = acc[k];
+                    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+                    if (lane == 0) s_w[warp][k] = x;
+                }
             }
             __syncthreads();
             if (threadIdx.x < d.n_open) {
                 double t = 0.0;
-                for (int w = 0; w < int(blockDim.x) / 32; ++w) t += s_w[w][threadIdx.x];
+                for (int w = 0; w < busy; ++w) t += s_w[w][threadIdx.x];
                 d.q_part[int64_t(bx) * MAX_OPEN + threadIdx.x] = t;
             }
         }
     }
 }
 
-template <int ST, int MODEL, bool GAL, bool FORCE>
+// A block of a single lattice's grid; the first is the clock, beside the node blocks.
+template <int ST, int MODEL, bool GAL, bool FORCE, bool OPEN>
+__device__ __forceinline__ void bulk_block(const cs_step_desc& d, const int a) {
+    if (blockIdx.x == 0) {
+        grid_dependency_wait();
+        if (threadIdx.x < 32) advance_clock(d, a);
+        launch_dependents();
+        return;
+    }
+    bulk_body<ST, MODEL, GAL, FORCE, OPEN>(d, a, int(blockIdx.x) - 1, false);
+}
+
+template <int ST, int MODEL, bool GAL, bool FORCE, bool OPEN>
 __global__ void __launch_bounds__(MAX_BLOCK, MIN_BLOCKS) k_bulk(const cs_step_desc d, const int a) {
-    bulk_body<ST, MODEL, GAL, FORCE>(d, a, blockIdx.x);
+    bulk_block<ST, MODEL, GAL, FORCE, OPEN>(d, a);
 }
 
 // The regularised step without a body force (every open vessel) in blocks of at most 128 threads: compiled for 9
@@ -744,34 +807,64 @@ __global__ void __launch_bounds__(MAX_BLOCK, MIN_BLOCKS) k_bulk(const cs_step_de
 constexpr int DENSE_BLOCK = 128;
 constexpr int DENSE_MIN_BLOCKS = 9;
 
+// (One build with and without open ends: at this register limit the one without their reduction spills 28 bytes, this
+// one 8, and takes 89 us a step on the 1.49 M-node artery against 86.)
 template <int ST, bool GAL>
 __global__ void __launch_bounds__(DENSE_BLOCK, DENSE_MIN_BLOCKS) k_bulk_dense(const cs_step_desc d, const int a) {
-    bulk_body<ST, CS_MODEL_REGULARISED, GAL, false>(d, a, blockIdx.x);
+    bulk_block<ST, CS_MODEL_REGULARISED, GAL, false, true>(d, a);
 }
 
 // ---- 3. outlet resistances ----------------------------------------------------------------------------------------
-constexpr int BC_THREADS = 256;
+constexpr int BC_THREADS = 512;
 
 // simulate.py:76-82 in FP64 (one block of BC_THREADS threads); the drive of this step was stored by the boundary
-// kernel. Q_k = the flux blocks' partial sums, added by a fixed-shape tree (the same order at every step and run).
+// kernel. Q_k = the flux blocks' partial sums: a thread adds its rows (all open ends of a row lie side by side), warps
+// reduce by shuffles and the warps' sums are added in order (the same order at every step and run). The kernel is pure
+// latency on the path from one step to the next: launched programmatically, it reads fb_list before the bulk kernel has
+// ended and lets the next boundary kernel become resident while it works. A tree over all threads per open end and an
+// ordinary launch took 8.3 us on 1487 rows, a quarter of a step of 190 k nodes.
 __device__ __forceinline__ void bc_body(const cs_step_desc& d) {
-    __shared__ double s_red[BC_THREADS];
-    __shared__ double s_q[MAX_OPEN];
-    for (int k = 0; k < d.n_open; ++k) {
-        double t = 0.0;
-        for (int j = threadIdx.x; j < d.n_fb; j += BC_THREADS) t += d.q_part[int64_t(__ldg(d.fb_list + j)) * MAX_OPEN + k];
-        s_red[threadIdx.x] = t;
-        __syncthreads();
-        for (int h = BC_THREADS / 2; h > 0; h >>= 1) {
-            if (threadIdx.x < h) s_red[threadIdx.x] += s_red[threadIdx.x + h];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) s_q[k] = s_red[0];
-        __syncthreads();
+    __shared__ double s_w[BC_THREADS / 32][MAX_OPEN];
+    constexpr int AHEAD = 4;
+    launch_dependents();
+    int32_t row[AHEAD];
+#pragma unroll
+    for (int r = 0; r < AHEAD; ++r) {
+        const int j = threadIdx.x + r * BC_THREADS;
+        row[r] = j < d.n_fb ? __ldg(d.fb_list + j) : -1;
     }
+    double acc[MAX_OPEN];
+#pragma unroll
+    for (int k = 0; k < MAX_OPEN; ++k) acc[k] = 0.0;
+    grid_dependency_wait();
+#pragma unroll
+    for (int k = 0; k < MAX_OPEN; ++k) {
+        if (k >= d.n_open) break;
+        double v[AHEAD];
+#pragma unroll
+        for (int r = 0; r < AHEAD; ++r) v[r] = row[r] >= 0 ? d.q_part[int64_t(row[r]) * MAX_OPEN + k] : 0.0;
+#pragma unroll
+        for (int r = 0; r < AHEAD; ++r) acc[k] += v[r];
+    }
+    for (int j = threadIdx.x + AHEAD * BC_THREADS; j < d.n_fb; j += BC_THREADS) {
+        const double* q = d.q_part + int64_t(__ldg(d.fb_list + j)) * MAX_OPEN;
+#pragma unroll
+        for (int k = 0; k < MAX_OPEN; ++k)
+            if (k < d.n_open) acc[k] += q[k];
+    }
+#pragma unroll
+    for (int k = 0; k < MAX_OPEN; ++k) {
+        if (k >= d.n_open) break;
+        double x = acc[k];
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5][k] = x;
+    }
+    __syncthreads();
     const int k = threadIdx.x;
     if (k >= d.n_open) return;
-    const double qk = s_q[k];
+    double qk = 0.0;
+#pragma unroll
+    for (int w = 0; w < BC_THREADS / 32; ++w) qk += s_w[w][k];
     d.q_last[k] = qk;
     double pk;
     if (k == 0) {
@@ -791,26 +884,27 @@ __device__ __forceinline__ void bc_body(const cs_step_desc& d) {
     }
 }
 
-__global__ void k_bc(const cs_step_desc d) { bc_body(d); }
+__global__ void __launch_bounds__(BC_THREADS) k_bc(const cs_step_desc d, const int) { bc_body(d); }
 
 using StepFn = void (*)(const cs_step_desc, const int);
 
-template <int ST>
-StepFn pick_force(int model, int gal, bool force, int block) {
-    if (model == CS_MODEL_REGULARISED && !force && block <= DENSE_BLOCK)
-        return gal ? k_bulk_dense<ST, true> : k_bulk_dense<ST, false>;
-    if (model == CS_MODEL_REGULARISED) {
-        if (gal) return force ? k_bulk<ST, CS_MODEL_REGULARISED, true, true> : k_bulk<ST, CS_MODEL_REGULARISED, true, false>;
-        return force ? k_bulk<ST, CS_MODEL_REGULARISED, false, true> : k_bulk<ST, CS_MODEL_REGULARISED, false, false>;
-    }
-    if (gal) return force ? k_bulk<ST, CS_MODEL_TRT, true, true> : k_bulk<ST, CS_MODEL_TRT, true, false>;
-    return force ? k_bulk<ST, CS_MODEL_TRT, false, true> : k_bulk<ST, CS_MODEL_TRT, false, false>;
+template <int ST, bool GAL, bool OPEN>
+StepFn pick_collision(int model, bool force, int block) {
+    if (model != CS_MODEL_REGULARISED)
+        return force ? k_bulk<ST, CS_MODEL_TRT, GAL, true, OPEN> : k_bulk<ST, CS_MODEL_TRT, GAL, false, OPEN>;
+    if (force) return k_bulk<ST, CS_MODEL_REGULARISED, GAL, true, OPEN>;
+    return block <= DENSE_BLOCK ? k_bulk_dense<ST, GAL> : k_bulk<ST, CS_MODEL_REGULARISED, GAL, false, OPEN>;
 }
 
 template <int ST>
 StepFn pick_model(const cs_step_desc& d) {
     const bool force = d.force[0] != 0.0f || d.force[1] != 0.0f || d.force[2] != 0.0f;
-    return pick_force<ST>(d.model, d.gal, force, d.block ? d.block : MAX_BLOCK);
+    const int block = d.block ? d.block : MAX_BLOCK;
+    if (d.n_open > 0)
+        return d.gal ? pick_collision<ST, true, true>(d.model, force, block)
+                     : pick_collision<ST, false, true>(d.model, force, block);
+    return d.gal ? pick_collision<ST, true, false>(d.model, force, block)
+                 : pick_collision<ST, false, false>(d.model, force, block);
 }
 
 StepFn pick_bulk(const cs_step_desc& d) {
@@ -829,11 +923,19 @@ StepFn pick_boundary(const cs_step_desc& d) {
     }
 }
 
-int validate(const cs_step_desc* d) {
-    if (!d) return fail(CS_ERR_ARG, "cs_step: null descriptor");
+cs_step_desc with_strides(const cs_step_desc& d);
+
+int validate(const cs_step_desc* user) {
+    if (!user) return fail(CS_ERR_ARG, "cs_step: null descriptor");
+    const cs_step_desc filled = with_strides(*user);
+    const cs_step_desc* d = &filled;
     if (d->n < 0 || d->n >= (int64_t(1) << 30)) return fail(CS_ERR_SIZE, "cs_step: n = %lld", (long long)d->n);
     if (d->gmax < 0 || d->npad != d->n + d->gmax || int64_t(Q) * d->npad >= (int64_t(1) << 31))
         return fail(CS_ERR_SIZE, "cs_step: npad %lld must be n + gmax with 27 * npad < 2^31", (long long)d->npad);
+    if (d->fstride < d->npad || int64_t(Q) * d->fstride >= (int64_t(1) << 31) || d->vstride < d->n ||
+        3 * d->vstride >= (int64_t(1) << 31))
+        return fail(CS_ERR_SIZE, "cs_step: row strides %lld (npad %lld; 27 rows below 2^31) and %lld (n %lld)",
+                    (long long)d->fstride, (long long)d->npad, (long long)d->vstride, (long long)d->n);
     if (d->gblock[0] != 0) return fail(CS_ERR_ARG, "cs_step: gblock[0] = %d", d->gblock[0]);
     for (int i = 0; i < Q; ++i) {
         const int64_t w = int64_t(d->gblock[i + 1]) - d->gblock[i];
@@ -846,7 +948,7 @@ int validate(const cs_step_desc* d) {
     if (d->block != 0 && (d->block < 32 || d->block > MAX_BLOCK || d->block % 32))
         return fail(CS_ERR_ARG, "cs_step: block %d (32..%d, multiple of 32)", d->block, MAX_BLOCK);
     if (d->period < 1 || d->nh < 0 || d->ramp < 0) return fail(CS_ERR_ARG, "cs_step: period %d nh %d ramp %d", d->period, d->nh, d->ramp);
-    if (!d->tick || !d->drive || !d->coef || !d->p_out || d->n_out < 1)
+    if (!d->tick || !d->drive || !d->drive2 || !d->coef || !d->p_out || d->n_out < 1)
         return fail(CS_ERR_ARG, "cs_step: null clock / outlet state");
     if (d->n > 0 && (!d->f[0] || !d->f[1] || !d->vel[0] || !d->vel[1] || !d->rho || !d->lcode || !d->uin || !d->om))
         return fail(CS_ERR_ARG, "cs_step: null lattice buffer");
@@ -857,6 +959,34 @@ int validate(const cs_step_desc* d) {
                           d->n_fb < 0 || (d->n_fb > 0 && !d->fb_list) ||
                           (d->n_flux > 0 && (!d->flux_idx || !d->flux_w || !d->flux_slot))))
         return fail(CS_ERR_ARG, "cs_step: null flux buffer");
+    return CS_OK;
+}
+
+// A descriptor with its row strides filled in (0: rows back to back).
+cs_step_desc with_strides(const cs_step_desc& d) {
+    cs_step_desc r = d;
+    if (r.fstride == 0) r.fstride = r.npad;
+    if (r.vstride == 0) r.vstride = r.n;
+    return r;
+}
+
+// One division of the SM's memory between L1 and shared memory for every kernel of a step. By default the driver picks
+// it by each kernel's own shared memory (none in the boundary kernel, 9 blocks x 4.6 KB in the bulk kernel), and an SM
+// that changes it between two kernels drains first: the next kernel's blocks then do not start under the last one's
+// (20 k-node cylinder 9.6 us a step, with one division 5.0; tilted pipe of 75 k nodes 12.6 and 8.4). 28 % is the 64 KB
+// that nine blocks of the bulk kernel need; half of it leaves room for seven (artery 88.6 against 86.5 us).
+constexpr int CARVEOUT = 28;
+
+int set_carveout(const void* fn) {
+    static std::mutex m;
+    static std::vector<std::pair<int, const void*>> done;
+    int dev = 0;
+    CS_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(m);
+    const std::pair<int, const void*> key(dev, fn);
+    if (std::find(done.begin(), done.end(), key) != done.end()) return CS_OK;
+    CS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, CARVEOUT));
+    done.push_back(key);
     return CS_OK;
 }
 
@@ -877,23 +1007,37 @@ int launch_pdl(StepFn fn, dim3 grid, dim3 block, cudaStream_t st, const cs_step_
     return CS_OK;
 }
 
-int launch_steps(const cs_step_desc* d, int a, int steps, cudaStream_t st) {
+int launch_steps(const cs_step_desc* user, int a, int steps, cudaStream_t st) {
+    const cs_step_desc filled = with_strides(*user);
+    const cs_step_desc* d = &filled;
     const int block = d->block ? d->block : MAX_BLOCK;
     const unsigned grid = unsigned(d->n > 0 ? ceil_div(d->n, block) : 0);
     const dim3 bgrid(unsigned(boundary_items(*d)));
     StepFn bulk = pick_bulk(*d);
     StepFn bound = pick_boundary(*d);
-    for (int s = 0; s < steps; ++s) {
-        // always launched: it also advances the clock
-        int rc = launch_pdl(bound, bgrid, dim3(B_THREADS), st, *d, a);
+    for (StepFn fn : {bulk, bound, StepFn(k_bc), StepFn(k_clock)}) {
+        const int rc = set_carveout(reinterpret_cast<const void*>(fn));
         if (rc != CS_OK) return rc;
-        if (grid > 0) {
-            rc = launch_pdl(bulk, dim3(grid), dim3(block), st, *d, a);
+    }
+    if (steps > 0 && grid > 0) {
+        k_clock<<<1, 32, 0, st>>>(*d, a);
+        CS_CHECK_LAUNCH("k_clock");
+    }
+    for (int s = 0; s < steps; ++s) {
+        int rc = CS_OK;
+        if (grid == 0) {
+            k_clock<<<1, 32, 0, st>>>(*d, a);
+            k_clock_only<<<1, 32, 0, st>>>(*d, a);
+            CS_CHECK_LAUNCH("k_clock_only");
+        } else {
+            if (d->gmax > 0) rc = launch_pdl(bound, bgrid, dim3(B_THREADS), st, *d, a);
+            if (rc != CS_OK) return rc;
+            rc = launch_pdl(bulk, dim3(grid + 1), dim3(block), st, *d, a);
             if (rc != CS_OK) return rc;
         }
         if (d->n_open > 0) {
-            k_bc<<<1, BC_THREADS, 0, st>>>(*d);
-            CS_CHECK_LAUNCH("k_bc");
+            rc = launch_pdl(k_bc, dim3(1), dim3(BC_THREADS), st, *d, a);
+            if (rc != CS_OK) return rc;
         }
         a = 1 - a;
     }
@@ -1055,7 +1199,7 @@ __global__ void __launch_bounds__(B_THREADS) k_boundary_batch(const __grid_const
 // more of them. The claim for the following item is issued at the start of the current one and lands while it
 // runs. Which block updates which item does not change any result (each item writes its own nodes and its own row
 // of flux partial sums).
-template <int ST, int MODEL, bool GAL, bool FORCE>
+template <int ST, int MODEL, bool GAL, bool FORCE, bool OPEN>
 __global__ void __launch_bounds__(MAX_BLOCK, MIN_BLOCKS) k_bulk_batch(const __grid_constant__ BatchGroup g,
                                                                       const int a) {
     __shared__ int s_item[2];
@@ -1066,7 +1210,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, MIN_BLOCKS) k_bulk_batch(const __gr
         const int local = cur.next(item);
         int claim = 0;
         if (!first && threadIdx.x == 0) claim = atomicAdd(g.counter, 1);
-        bulk_body<ST, MODEL, GAL, FORCE>(g.d[cur.inst], a ^ g.parity[cur.inst], local);
+        bulk_body<ST, MODEL, GAL, FORCE, OPEN>(g.d[cur.inst], a ^ g.parity[cur.inst], local, local == 0);
         if (first && threadIdx.x == 0) claim = atomicAdd(g.counter, 1);   // after the wait inside bulk_body
         first = false;
         if (threadIdx.x == 0) s_item[buf] = int(gridDim.x) + claim;
@@ -1079,31 +1223,51 @@ __global__ void __launch_bounds__(MAX_BLOCK, MIN_BLOCKS) k_bulk_batch(const __gr
 // One block per bulk item, no loop and no claims (grid_bulk = 0): the regularised step without body force in blocks
 // of at most 128 threads, compiled like k_bulk_dense for 9 blocks per SM, which the persistent loop's state does not
 // leave registers for. The block finds its instance by a binary search over the item prefix in the parameters.
-template <int ST, bool GAL>
+template <int ST, bool GAL, bool OPEN>
 __global__ void __launch_bounds__(DENSE_BLOCK, DENSE_MIN_BLOCKS) k_bulk_batch_dense(const __grid_constant__ BatchGroup g,
                                                                                   const int a) {
     const int item = int(blockIdx.x);
     const int inst = find_instance(g.bulk_prefix, g.n_inst, item);
-    bulk_body<ST, CS_MODEL_REGULARISED, GAL, false>(g.d[inst], a ^ g.parity[inst], item - g.bulk_prefix[inst]);
+    const int local = item - g.bulk_prefix[inst];
+    bulk_body<ST, CS_MODEL_REGULARISED, GAL, false, OPEN>(g.d[inst], a ^ g.parity[inst], local, local == 0);
 }
 
-__global__ void k_bc_batch(const __grid_constant__ BatchGroup g) {
+__global__ void __launch_bounds__(32) k_clock_batch(const __grid_constant__ BatchGroup g, const int a) {
+    first_clock(g.d[blockIdx.x], a ^ g.parity[blockIdx.x]);
+}
+
+// The instances without nodes, whose clock no bulk block advances.
+__global__ void __launch_bounds__(32) k_clock_empty_batch(const __grid_constant__ BatchGroup g, const int a) {
+    if (g.d[blockIdx.x].n == 0) advance_clock(g.d[blockIdx.x], a ^ g.parity[blockIdx.x]);
+}
+
+__global__ void __launch_bounds__(BC_THREADS) k_bc_batch(const __grid_constant__ BatchGroup g, const int) {
     const cs_step_desc& d = g.d[blockIdx.x];
-    if (d.n_open > 0) bc_body(d);
+    if (d.n_open > 0) {
+        bc_body(d);
+    } else {
+        grid_dependency_wait();     // the next boundary kernel waits for this one, and through it for the bulk kernel
+    }
 }
 
 using BatchFn = void (*)(const BatchGroup, const int);
 
+template <int ST, bool GAL, bool OPEN>
+BatchFn pick_batch_collision(int model, bool force, bool dense) {
+    if (model != CS_MODEL_REGULARISED)
+        return force ? k_bulk_batch<ST, CS_MODEL_TRT, GAL, true, OPEN> : k_bulk_batch<ST, CS_MODEL_TRT, GAL, false, OPEN>;
+    if (force) return k_bulk_batch<ST, CS_MODEL_REGULARISED, GAL, true, OPEN>;
+    return dense ? k_bulk_batch_dense<ST, GAL, OPEN> : k_bulk_batch<ST, CS_MODEL_REGULARISED, GAL, false, OPEN>;
+}
+
 template <int ST>
-BatchFn pick_batch_model(int model, int gal, bool force, bool dense) {
-    if (dense && model == CS_MODEL_REGULARISED && !force)
-        return gal ? k_bulk_batch_dense<ST, true> : k_bulk_batch_dense<ST, false>;
-    if (model == CS_MODEL_REGULARISED) {
-        if (gal) return force ? k_bulk_batch<ST, CS_MODEL_REGULARISED, true, true> : k_bulk_batch<ST, CS_MODEL_REGULARISED, true, false>;
-        return force ? k_bulk_batch<ST, CS_MODEL_REGULARISED, false, true> : k_bulk_batch<ST, CS_MODEL_REGULARISED, false, false>;
-    }
-    if (gal) return force ? k_bulk_batch<ST, CS_MODEL_TRT, true, true> : k_bulk_batch<ST, CS_MODEL_TRT, true, false>;
-    return force ? k_bulk_batch<ST, CS_MODEL_TRT, false, true> : k_bulk_batch<ST, CS_MODEL_TRT, false, false>;
+BatchFn pick_batch_model(const cs_batch_desc& b, bool dense) {
+    const bool force = b.force != 0;
+    if (b.any_open)
+        return b.gal ? pick_batch_collision<ST, true, true>(b.model, force, dense)
+                     : pick_batch_collision<ST, false, true>(b.model, force, dense);
+    return b.gal ? pick_batch_collision<ST, true, false>(b.model, force, dense)
+                 : pick_batch_collision<ST, false, false>(b.model, force, dense);
 }
 
 int validate_batch(const cs_batch_desc* b) {
@@ -1147,7 +1311,7 @@ std::vector<BatchGroup> make_groups(const cs_batch_desc* b) {
         g.counter = b->counter + i0 / CS_BATCH_GROUP;
         int64_t bulk = 0, bnd = 0;
         for (int k = 0; k < g.n_inst; ++k) {
-            const cs_step_desc& d = b->descs[i0 + k];
+            const cs_step_desc d = with_strides(b->descs[i0 + k]);
             g.d[k] = d;
             g.parity[k] = b->parity[i0 + k];
             g.bulk_prefix[k] = int32_t(bulk);
@@ -1181,15 +1345,30 @@ int launch_batch_pdl(BatchFn fn, unsigned grid, unsigned block, cudaStream_t st,
 
 int launch_batch(const cs_batch_desc* b, int a, int steps, cudaStream_t st) {
     const std::vector<BatchGroup> gs = make_groups(b);
-    const bool force = b->force != 0;
     const bool dense = b->grid_bulk == 0 && b->block <= DENSE_BLOCK;     // one block per item: k_bulk_batch_dense
-    BatchFn bulk = b->storage == CS_STORE_F16    ? pick_batch_model<CS_STORE_F16>(b->model, b->gal, force, dense)
-                   : b->storage == CS_STORE_BF16 ? pick_batch_model<CS_STORE_BF16>(b->model, b->gal, force, dense)
-                                                 : pick_batch_model<CS_STORE_F32>(b->model, b->gal, force, dense);
+    BatchFn bulk = b->storage == CS_STORE_F16    ? pick_batch_model<CS_STORE_F16>(*b, dense)
+                   : b->storage == CS_STORE_BF16 ? pick_batch_model<CS_STORE_BF16>(*b, dense)
+                                                 : pick_batch_model<CS_STORE_F32>(*b, dense);
     BatchFn bound = b->storage == CS_STORE_F16    ? k_boundary_batch<CS_STORE_F16>
                     : b->storage == CS_STORE_BF16 ? k_boundary_batch<CS_STORE_BF16>
                                                   : k_boundary_batch<CS_STORE_F32>;
+    for (BatchFn fn : {bulk, bound, BatchFn(k_bc_batch), BatchFn(k_clock_batch), BatchFn(k_clock_empty_batch)}) {
+        const int rc = set_carveout(reinterpret_cast<const void*>(fn));
+        if (rc != CS_OK) return rc;
+    }
+    bool empty = false;
+    for (int i = 0; i < b->n_inst; ++i) empty = empty || b->descs[i].n == 0;
+    if (steps > 0)
+        for (const BatchGroup& g : gs) {
+            k_clock_batch<<<unsigned(g.n_inst), 32, 0, st>>>(g, a);
+            CS_CHECK_LAUNCH("k_clock_batch");
+        }
     for (int s = 0; s < steps; ++s) {
+        if (empty)
+            for (const BatchGroup& g : gs) {
+                k_clock_empty_batch<<<unsigned(g.n_inst), 32, 0, st>>>(g, a);
+                CS_CHECK_LAUNCH("k_clock_empty_batch");
+            }
         for (const BatchGroup& g : gs) {
             const unsigned gb = unsigned(b->grid_bnd > 0 ? std::min(b->grid_bnd, g.bnd_items) : g.bnd_items);
             const int rc = launch_batch_pdl(bound, gb, B_THREADS, st, g, a);
@@ -1203,8 +1382,8 @@ int launch_batch(const cs_batch_desc* b, int a, int steps, cudaStream_t st) {
         }
         if (b->any_open) {
             for (const BatchGroup& g : gs) {
-                k_bc_batch<<<unsigned(g.n_inst), BC_THREADS, 0, st>>>(g);
-                CS_CHECK_LAUNCH("k_bc_batch");
+                const int rc = launch_batch_pdl(k_bc_batch, unsigned(g.n_inst), BC_THREADS, st, g, a);
+                if (rc != CS_OK) return rc;
             }
         }
         a = 1 - a;

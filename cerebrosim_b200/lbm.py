@@ -205,6 +205,16 @@ def _upload(x, dtype, dev):
     return torch.as_tensor(np.ascontiguousarray(x, np_dtype)).to(dev)
 
 
+def _line_rows(rows, cols, dtype, dev):
+    """Zeros of shape (rows, cols) whose rows start on 128-byte lines: the step's stores then split no sector at the
+    ends of a warp (27 FP16 rows streamed: 34.9 against 38.0 us for 1.49 M nodes; FP32 53.7 against 56.8)."""
+    line = 128 // torch.empty(0, dtype=dtype).element_size()
+    stride = -(-cols // line) * line
+    if rows * stride >= 1 << 31:             # the step's 32-bit offsets: the last few sizes keep their rows back to back
+        stride = cols
+    return torch.zeros((rows, stride), dtype=dtype, device=dev)[:, :cols]
+
+
 def _ptr(t):
     return ctypes.c_void_p(t.data_ptr()) if t is not None and t.numel() else None
 
@@ -321,8 +331,8 @@ class Solver:
             setup.synchronize()
             del scratch
             self.links = None                          # the full 27 x N table is not needed by the step
-            self.f = [torch.zeros((Q, self.npad), dtype=pop_dtype, device=dev) for _ in range(2)]
-            self.vel = [torch.zeros((3, N), dtype=torch.float32, device=dev) for _ in range(2)]
+            self.f = [_line_rows(Q, self.npad, pop_dtype, dev) for _ in range(2)]
+            self.vel = [_line_rows(3, N, torch.float32, dev) for _ in range(2)]
             self.vels = [v.T for v in self.vel]
             self.rho = torch.zeros(N, dtype=torch.float32, device=dev)
             self.p_out = torch.zeros(n_out, dtype=torch.float32, device=dev)
@@ -332,9 +342,10 @@ class Solver:
             self.om = torch.full((N,), 1.0 / self.tau, dtype=torch.float32, device=dev) * self._om_sign
             self.tick = torch.zeros(2, dtype=torch.int32, device=dev)
             self.drv = torch.zeros(1, dtype=torch.float32, device=dev)
+            self._drv2 = torch.zeros(2, dtype=torch.float32, device=dev)
             for t in (self.perm, self.inv, self.uin, self.inl, self.gnode, self.ginfo, self.gq, self.lcode,
                       self.segdelta, self.irr, *self.f, *self.vel, self.rho, self.p_out, self.p_out64,
-                      self._om_sign, self.om, self.tick, self.drv):
+                      self._om_sign, self.om, self.tick, self.drv, self._drv2):
                 if t is not None:
                     t.record_stream(self.stream)
             self.stream.wait_stream(setup)
@@ -443,6 +454,8 @@ class Solver:
         d.tick, d.drive, d.coef = self.tick.data_ptr(), self.drv.data_ptr(), self.coef.data_ptr()
         d.nh, d.period, d.ramp = self.nh, self.period, self.ramp
         d.p_out64 = self.p_out64.data_ptr()
+        d.drive2 = self._drv2.data_ptr()
+        d.fstride, d.vstride = self.f[0].stride(0), self.vel[0].stride(0)
         self._fill_desc(d)
         return d
 

@@ -186,7 +186,7 @@ class Probes:
         s = self.s
         with torch.cuda.device(s.dev), torch.cuda.stream(s.stream):
             check(_lib.load().cs_probe_gather(ctypes_void(s.rho.data_ptr()), ctypes_void(s.vel[s.cur].data_ptr()),
-                                              s.N, ctypes_void(self.cells.data_ptr()),
+                                              s.vel[s.cur].stride(0), ctypes_void(self.cells.data_ptr()),
                                               ctypes_void(self.start.data_ptr()), self.n,
                                               ctypes_void(self.psum.data_ptr()), ctypes_void(self.umax.data_ptr()),
                                               ctypes_void(s.stream.cuda_stream)))
@@ -225,8 +225,8 @@ class CoarseMap:
     def frame(self):
         s = self.s
         with torch.cuda.device(s.dev), torch.cuda.stream(s.stream):
-            check(_lib.load().cs_bin_fields(ctypes_void(s.rho.data_ptr()), ctypes_void(s.vel[s.cur].data_ptr()), s.N,
-                                            ctypes_void(self.cells.data_ptr()), ctypes_void(self.start.data_ptr()),
+            check(_lib.load().cs_bin_fields(ctypes_void(s.rho.data_ptr()), ctypes_void(s.vel[s.cur].data_ptr()),
+                                            s.vel[s.cur].stride(0), ctypes_void(self.cells.data_ptr()), ctypes_void(self.start.data_ptr()),
                                             self.n_bins, ctypes_void(self.p.data_ptr()), ctypes_void(self.u.data_ptr()),
                                             ctypes_void(s.stream.cuda_stream)))
         s.stream.synchronize()

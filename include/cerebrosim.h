@@ -183,8 +183,8 @@ typedef struct cs_step_desc {
     float magic;             /* TRT magic parameter */
     float force[3];          /* body force, scaled by the drive */
     int32_t block;           /* threads per block of the bulk kernel; 0 = default */
-    void* f[2];              /* populations (27 * npad) in `storage` format, link-major */
-    float* vel[2];           /* velocity, SoA: vel[b][c * n + node] */
+    void* f[2];              /* populations (27 rows of npad, fstride apart) in `storage` format, link-major */
+    float* vel[2];           /* velocity, SoA: vel[b][c * vstride + node] */
     float* rho;              /* density deviation (n) */
     const int32_t* lcode;    /* compressed connectivity (n) from cs_compress_fill */
     const int32_t* segdelta; /* (CS_SEG_STRIDE * n_seg), 16-byte aligned */
@@ -223,6 +223,11 @@ typedef struct cs_step_desc {
      * beat_acc[k] and q_last[k] to beat_acc[n_open + k] (FP64) and 1 to beat_acc[2 * n_open]; the caller zeroes
      * it at a beat's start and divides by the count at its end (the beat means of simulate.py:325-333). */
     double* beat_acc;
+    float* drive2;           /* (2): the drive of the step that reads buffer a, written by the step before it, and for
+                              * the first step of a call by a one-warp kernel */
+    int64_t fstride;         /* elements between population rows, >= npad, 27 * fstride < 2^31; 0: npad. Rows that start
+                              * on a 128-byte line cost the kernel's stores no split sectors */
+    int64_t vstride;         /* elements between velocity rows, >= n; 0: n */
 } cs_step_desc;
 
 /* Block partition of a sorted flux list for `block` threads per block: out[b] = first entry with
@@ -283,8 +288,8 @@ int cs_wss_shear(const float* U, int64_t n_cells, const int32_t* idx, const floa
 
 /* ---------------------------------------------------------------------------------------------------------------
  * Heartbeat-loop measurements — replace simulate.k_gather (simulate.py:85-90) and the coarse-map averaging of the
- * stored frames (simulate.py:236-242, 346-353). rho (n) and vel (SoA, 3 * n) are a solver's state buffers; `cells`
- * lists cell indices (each < n, checked by the caller) grouped by segment, `start` (segments + 1) delimits them.
+ * stored frames (simulate.py:236-242, 346-353). rho and vel (three rows, n elements apart) are a solver's state
+ * buffers; `cells` lists cell indices (each a node, checked by the caller) grouped by segment, `start` (segments + 1) delimits them.
  * Sums are FP64 in a fixed order.
  * ------------------------------------------------------------------------------------------------------------- */
 
