@@ -22,8 +22,8 @@
 //     keeps the populations.
 //     Its first block is the clock (lbm.py:94-102): it stores this step's drive, advances tick[1 - a] = tick[a] + 1 and
 //     evaluates the next step's drive.
-//  3. k_bc (only with the resistance coupling) — one block, launched programmatically too: p_out[0] = drive, p_out[k] relaxed towards R_k Q_k -
-//     pref in FP64, Qlast = Q, Q = 0 (simulate.py:76-82). The slab flux Q_k = sum u . w itself is reduced in the
+//  3. k_bc (only with the resistance coupling) — one block: p_out[0] = drive, p_out[k] relaxed towards R_k Q_k - pref
+//     in FP64, Qlast = Q, Q = 0 (simulate.py:76-82). The slab flux Q_k = sum u . w itself is reduced in the
 //     bulk kernel in FP64 by the blocks that hold flux cells (simulate.py:65-69).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -57,12 +57,35 @@ __device__ __forceinline__ float scale_rt(int i) {
 }
 
 // ---- population storage -----------------------------------------------------------------------------------------
-// 32-bit element offsets: 27 * fstride < 2^31 is checked on the host.
+// A population that its reader will not need again: out of the caches first. Volatile, as the wait it must stay behind.
+__device__ __forceinline__ float ld_first(const float* p) {
+    float v;
+    asm volatile("ld.global.nc.L1::evict_first.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ __half ld_first(const __half* p) {
+    unsigned short v;
+    asm volatile("ld.global.nc.L1::evict_first.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    return __ushort_as_half(v);
+}
+__device__ __forceinline__ __nv_bfloat16 ld_first(const __nv_bfloat16* p) {
+    unsigned short v;
+    asm volatile("ld.global.nc.L1::evict_first.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    return __ushort_as_bfloat16(v);
+}
+template <bool FIRST, class T>
+__device__ __forceinline__ T ld_pop(const T* p) {
+    if constexpr (FIRST) return ld_first(p);
+    else return __ldg(p);
+}
+
+// 32-bit element offsets: 27 * fstride < 2^31 is checked on the host. FIRST: ld_first (see k_bulk_dense).
 template <int ST> struct Pop;
 
 template <> struct Pop<CS_STORE_F32> {
+    template <bool FIRST = false>
     static __device__ __forceinline__ float ld(const void* b, uint32_t idx, float) {
-        return __ldg(static_cast<const float*>(b) + idx);
+        return ld_pop<FIRST>(static_cast<const float*>(b) + idx);
     }
     static __device__ __forceinline__ void st(void* b, uint32_t idx, float, float v) { static_cast<float*>(b)[idx] = v; }
     static __device__ __forceinline__ void st_link(void* b, uint32_t idx, int, float v) { static_cast<float*>(b)[idx] = v; }
@@ -71,8 +94,9 @@ template <> struct Pop<CS_STORE_F32> {
 // 16-bit formats store (f - w_i) * 1024 / w_i: all links share one range, well inside FP16's normal numbers, so the
 // relative rounding error is the format's 2^-11 (FP16) or 2^-8 (BF16) on every link. w is the link's weight.
 template <> struct Pop<CS_STORE_F16> {
+    template <bool FIRST = false>
     static __device__ __forceinline__ float ld(const void* b, uint32_t idx, float w) {
-        return __half2float(__ldg(static_cast<const __half*>(b) + idx)) * (w * (1.0f / 1024.0f));
+        return __half2float(ld_pop<FIRST>(static_cast<const __half*>(b) + idx)) * (w * (1.0f / 1024.0f));
     }
     static __device__ __forceinline__ void st(void* b, uint32_t idx, float w, float v) {
         static_cast<__half*>(b)[idx] = __float2half_rn(v * (1024.0f / w));
@@ -88,8 +112,9 @@ template <> struct Pop<CS_STORE_F16> {
 };
 
 template <> struct Pop<CS_STORE_BF16> {
+    template <bool FIRST = false>
     static __device__ __forceinline__ float ld(const void* b, uint32_t idx, float w) {
-        return __bfloat162float(__ldg(static_cast<const __nv_bfloat16*>(b) + idx)) * (w * (1.0f / 1024.0f));
+        return __bfloat162float(ld_pop<FIRST>(static_cast<const __nv_bfloat16*>(b) + idx)) * (w * (1.0f / 1024.0f));
     }
     static __device__ __forceinline__ void st(void* b, uint32_t idx, float w, float v) {
         static_cast<__nv_bfloat16*>(b)[idx] = __float2bfloat16_rn(v * (1024.0f / w));
@@ -104,18 +129,8 @@ template <> struct Pop<CS_STORE_BF16> {
 };
 
 // ---- helpers ------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ float drive_value(const cs_step_desc& d, int t) {
-    // lbm.py:95-100, float32
-    float ph = 2.0f * PI_F * float(t % d.period) / float(d.period);
-    float v = d.coef[0];
-    for (int k = 1; k <= d.nh; ++k)
-        v += d.coef[2 * k - 1] * cosf(float(k) * ph) + d.coef[2 * k] * sinf(float(k) * ph);
-    if (t < d.ramp) v *= 0.5f - 0.5f * cosf(PI_F * float(t) / float(d.ramp));
-    return v;
-}
-
-// The same by a whole warp, each lane one term's sine or cosine: a thread alone waits for its coefficients from memory one
-// harmonic after the other (4 us for three).
+// drive(t) (lbm.py:95-100, float32) by a whole warp, each lane one term's sine or cosine: a thread alone waits for its
+// coefficients from memory one harmonic after the other (4 us for three).
 __device__ __forceinline__ float drive_value_warp(const cs_step_desc& d, int t) {
     const int lane = threadIdx.x & 31;
     const float ph = 2.0f * PI_F * float(t % d.period) / float(d.period);
@@ -512,7 +527,7 @@ __device__ __forceinline__ void store_pairs(void* fout, uint32_t NP, int32_t n, 
     });
 }
 
-template <int ST, int MODEL, bool GAL, bool FORCE>
+template <int ST, int MODEL, bool GAL, bool FORCE, bool FIRST>
 __device__ __forceinline__ void node_update(const cs_step_desc& d, int a, int32_t n, float& ux_o, float& uy_o,
                                             float& uz_o) {
     const int32_t N = int32_t(d.n), NV = int32_t(d.vstride);
@@ -557,7 +572,7 @@ __device__ __forceinline__ void node_update(const cs_step_desc& d, int a, int32_
     float fk[Q];
     Unroll<0, Q>::run([&](auto ic) {
         constexpr int I = decltype(ic)::value;
-        fk[I] = Pop<ST>::ld(fin, uint32_t(I) * NP + uint32_t(lk[I]), wgt(I));
+        fk[I] = Pop<ST>::template ld<FIRST>(fin, uint32_t(I) * NP + uint32_t(lk[I]), wgt(I));
     });
     moments27(fk, m);
 
@@ -723,14 +738,14 @@ __device__ __forceinline__ void node_update(const cs_step_desc& d, int a, int32_
 // Block bx of a lattice's bulk grid (nodes bx * blockDim .. + blockDim - 1). Called by every thread of the block.
 // OPEN: the lattice may have open ends (n_open > 0); compiled apart for the kernels that lose by carrying their
 // reduction. clock: this block also advances the clock.
-template <int ST, int MODEL, bool GAL, bool FORCE, bool OPEN>
+template <int ST, int MODEL, bool GAL, bool FORCE, bool OPEN, bool FIRST = false>
 __device__ __forceinline__ void bulk_body(const cs_step_desc& d, const int a, const int bx, const bool clock) {
     const int32_t n0 = int32_t(bx) * int32_t(blockDim.x);
     const int32_t n = n0 + int32_t(threadIdx.x);
     // read after the update: bring the line in meanwhile, at the cost of no register
     if (OPEN && d.n_open > 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(d.flux_block + bx));
     float ux = 0.f, uy = 0.f, uz = 0.f;
-    if (n < d.n) node_update<ST, MODEL, GAL, FORCE>(d, a, n, ux, uy, uz);
+    if (n < d.n) node_update<ST, MODEL, GAL, FORCE, FIRST>(d, a, n, ux, uy, uz);
     grid_dependency_wait();      // (threads without a node) the flux accumulators were reset by the last step
     launch_dependents();
     if (clock && threadIdx.x < 32) advance_clock(d, a);
@@ -784,7 +799,7 @@ __device__ __forceinline__ void bulk_body(const cs_step_desc& d, const int a, co
 }
 
 // A block of a single lattice's grid; the first is the clock, beside the node blocks.
-template <int ST, int MODEL, bool GAL, bool FORCE, bool OPEN>
+template <int ST, int MODEL, bool GAL, bool FORCE, bool OPEN, bool FIRST = false>
 __device__ __forceinline__ void bulk_block(const cs_step_desc& d, const int a) {
     if (blockIdx.x == 0) {
         grid_dependency_wait();
@@ -792,7 +807,7 @@ __device__ __forceinline__ void bulk_block(const cs_step_desc& d, const int a) {
         launch_dependents();
         return;
     }
-    bulk_body<ST, MODEL, GAL, FORCE, OPEN>(d, a, int(blockIdx.x) - 1, false);
+    bulk_body<ST, MODEL, GAL, FORCE, OPEN, FIRST>(d, a, int(blockIdx.x) - 1, false);
 }
 
 template <int ST, int MODEL, bool GAL, bool FORCE, bool OPEN>
@@ -800,18 +815,23 @@ __global__ void __launch_bounds__(MAX_BLOCK, MIN_BLOCKS) k_bulk(const cs_step_de
     bulk_block<ST, MODEL, GAL, FORCE, OPEN>(d, a);
 }
 
-// The regularised step without a body force (every open vessel) in blocks of at most 128 threads: compiled for 9
-// such blocks per SM (56 registers, 8 bytes of spill) instead of 8 at 64 registers. The extra warps hide more of the
-// pulls' latency: 3-4 % faster steps from a cold L2 (the batched kernel, whose descriptor handling needs the
-// registers, keeps 64).
+// The regularised step without a body force (every open vessel) in blocks of at most 128 threads, compiled for as many
+// of them per SM as hide the pulls' latency best: 8 at 64 registers in FP32 (artery 79.6 us a step against 80.5 for 9 at
+// 56, 190 k-node artery 9.9 against 10.6), 9 at 56 in the 16-bit formats (67.4 against 67.6). The batched kernel, whose
+// descriptor handling needs the registers, keeps 64. (One build with and without open ends: at 56 registers the one
+// without their reduction spills 28 bytes, this one 8, and takes 89 us a step on the artery against 86.)
+//
+// FIRST: a step reads a population once, writes it to the other buffer, and a step later that copy is what is read: with
+// both buffers about as large as the L2, lines that have been read must go before lines just written. Loads marked so
+// take the 347 k-node FP32 pipe (75 MB) from 20.4 to 18.1 us a step, 522 k nodes (113 MB) from 29.4 to 27.2, 678 k nodes
+// in FP16 (73 MB) from 31.7 to 27.5. Past the L2 they lose the sectors that neighbouring warps share: 678 k nodes in FP32
+// (146 MB) 36.4 to 37.5, the artery (322 MB) 79.6 to 86.1. So the line is the L2's size.
 constexpr int DENSE_BLOCK = 128;
-constexpr int DENSE_MIN_BLOCKS = 9;
+constexpr int dense_blocks(int st) { return st == CS_STORE_F32 ? 8 : 9; }
 
-// (One build with and without open ends: at this register limit the one without their reduction spills 28 bytes, this
-// one 8, and takes 89 us a step on the 1.49 M-node artery against 86.)
-template <int ST, bool GAL>
-__global__ void __launch_bounds__(DENSE_BLOCK, DENSE_MIN_BLOCKS) k_bulk_dense(const cs_step_desc d, const int a) {
-    bulk_block<ST, CS_MODEL_REGULARISED, GAL, false, true>(d, a);
+template <int ST, bool GAL, bool FIRST>
+__global__ void __launch_bounds__(DENSE_BLOCK, dense_blocks(ST)) k_bulk_dense(const cs_step_desc d, const int a) {
+    bulk_block<ST, CS_MODEL_REGULARISED, GAL, false, true, FIRST>(d, a);
 }
 
 // ---- 3. outlet resistances ----------------------------------------------------------------------------------------
@@ -889,22 +909,32 @@ __global__ void __launch_bounds__(BC_THREADS) k_bc(const cs_step_desc d, const i
 using StepFn = void (*)(const cs_step_desc, const int);
 
 template <int ST, bool GAL, bool OPEN>
-StepFn pick_collision(int model, bool force, int block) {
+StepFn pick_collision(int model, bool force, int block, bool first) {
     if (model != CS_MODEL_REGULARISED)
         return force ? k_bulk<ST, CS_MODEL_TRT, GAL, true, OPEN> : k_bulk<ST, CS_MODEL_TRT, GAL, false, OPEN>;
     if (force) return k_bulk<ST, CS_MODEL_REGULARISED, GAL, true, OPEN>;
-    return block <= DENSE_BLOCK ? k_bulk_dense<ST, GAL> : k_bulk<ST, CS_MODEL_REGULARISED, GAL, false, OPEN>;
+    if (block <= DENSE_BLOCK) return first ? k_bulk_dense<ST, GAL, true> : k_bulk_dense<ST, GAL, false>;
+    return k_bulk<ST, CS_MODEL_REGULARISED, GAL, false, OPEN>;
+}
+
+// L2 bytes of the current device (0 if it cannot be asked: no kernel then assumes that anything fits).
+int64_t l2_bytes() {
+    int dev = 0, bytes = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&bytes, cudaDevAttrL2CacheSize, dev) != cudaSuccess) return 0;
+    return bytes;
 }
 
 template <int ST>
 StepFn pick_model(const cs_step_desc& d) {
     const bool force = d.force[0] != 0.0f || d.force[1] != 0.0f || d.force[2] != 0.0f;
     const int block = d.block ? d.block : MAX_BLOCK;
+    const bool first = 2 * int64_t(Q) * d.fstride * (ST == CS_STORE_F32 ? 4 : 2) <= l2_bytes();
     if (d.n_open > 0)
-        return d.gal ? pick_collision<ST, true, true>(d.model, force, block)
-                     : pick_collision<ST, false, true>(d.model, force, block);
-    return d.gal ? pick_collision<ST, true, false>(d.model, force, block)
-                 : pick_collision<ST, false, false>(d.model, force, block);
+        return d.gal ? pick_collision<ST, true, true>(d.model, force, block, first)
+                     : pick_collision<ST, false, true>(d.model, force, block, first);
+    return d.gal ? pick_collision<ST, true, false>(d.model, force, block, first)
+                 : pick_collision<ST, false, false>(d.model, force, block, first);
 }
 
 StepFn pick_bulk(const cs_step_desc& d) {
@@ -1224,7 +1254,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, MIN_BLOCKS) k_bulk_batch(const __gr
 // of at most 128 threads, compiled like k_bulk_dense for 9 blocks per SM, which the persistent loop's state does not
 // leave registers for. The block finds its instance by a binary search over the item prefix in the parameters.
 template <int ST, bool GAL, bool OPEN>
-__global__ void __launch_bounds__(DENSE_BLOCK, DENSE_MIN_BLOCKS) k_bulk_batch_dense(const __grid_constant__ BatchGroup g,
+__global__ void __launch_bounds__(DENSE_BLOCK, 9) k_bulk_batch_dense(const __grid_constant__ BatchGroup g,
                                                                                   const int a) {
     const int item = int(blockIdx.x);
     const int inst = find_instance(g.bulk_prefix, g.n_inst, item);

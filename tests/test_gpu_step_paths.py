@@ -1,0 +1,94 @@
+"""The step's paths beside its arithmetic, at the sizes where each can go wrong: the drive evaluated a step ahead, the
+flux sums over few and many blocks, population rows with and without padding, and an empty lattice's clock."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from cerebrosim_b200 import batch, cases, lbm, simulate  # noqa: E402
+
+
+def pipe(name="open_pipe_R8_L40"):
+    return lbm.build_lattice(**cases.lattice_args(cases.case(name)))
+
+
+def drive(coef, period, ramp, t):
+    ph = 2 * np.pi * (t % period) / period
+    k = np.arange(1, (len(coef) + 1) // 2)
+    v = coef[0] + (coef[1::2] * np.cos(k * ph) + coef[2::2] * np.sin(k * ph)).sum()
+    return v * (0.5 - 0.5 * np.cos(np.pi * t / ramp)) if t < ramp else v
+
+
+@pytest.mark.parametrize("harmonics", [0, 1, 16, 17, 33])
+def test_drive_of_every_step(harmonics):
+    """The drive stored by each step, over steps taken one by one, in one call and across a change of the drive, against
+    64 bits: float32 angles of up to 33 periods and a sum of 67 rounded terms stay within 33 * (2 pi * 33 * 2^-24) +
+    67 * 2^-24 < 5e-4 of terms below 1, here 1e-3."""
+    rng = np.random.default_rng(harmonics)
+    s = lbm.Solver(pipe(), 0.02, model="regularised")
+    t = 0
+    for coef, period, ramp in ((rng.uniform(-1, 1, 2 * harmonics + 1), 7, 5), (rng.uniform(-1, 1, 2 * harmonics + 1), 40, 0)):
+        coef = 1e-3 * coef
+        s.set_drive(coef, period=period, ramp=ramp)
+        for steps in (1, 1, 2, 5, 8):
+            s.run(steps, chunk=4)
+            t += steps
+            assert s.tick_value() == t
+            assert abs(s.drv.item() - drive(coef, period, ramp, t - 1)) < 5e-7
+
+
+@pytest.mark.parametrize("block", [32, 128, 256])
+@pytest.mark.parametrize("share", [0.0, 0.001, 1.0])
+def test_flux_sums(block, share):
+    """Flux over no cell, a few and every cell (77 k nodes in blocks of 32 are more rows than k_bc holds in flight)
+    equals the FP64 sum over the velocity field up to the rounding of 1e5 additions."""
+    lat = pipe("open_pipe_R16_L96")
+    n = lbm.n_nodes(lat)
+    rng = np.random.default_rng(3)
+    idx = np.flatnonzero(rng.uniform(size=n) < share)
+    flux = {"idx": idx, "w": rng.uniform(-1, 1, size=(len(idx), 3)).astype(np.float32), "slot": rng.integers(0, 1, len(idx))}
+    s = simulate.ArterySolver(lat, 0.02, flux, [0.0], 0.0, 0.1, model="regularised", block=block)
+    s.set_drive([0.02])
+    s.run(7)
+    u = s.fields()[1].astype(np.float64)
+    terms = (u[idx] * flux["w"]).sum(1)
+    assert abs(s.Qlast.numpy()[0] - terms.sum()) <= 1e5 * 2.0 ** -53 * np.abs(terms).sum()
+    assert s.p_out64[0].item() == s.drv.item()
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("kw", [{"model": "regularised"}, {"model": "trt"}, {"model": "regularised", "block": 256}])
+def test_padded_rows(storage, kw):
+    """Rows that start on 128-byte lines and rows back to back give the same fields bit for bit."""
+    lat = pipe("open_pipe_R7_L33")
+    out = []
+    for padded in (True, False):
+        s = lbm.Solver(lat, 0.02, storage=storage, **kw)
+        assert s.f[0].stride(0) * s.f[0].element_size() % 128 == 0 and s.vel[0].stride(0) % 32 == 0
+        if not padded:
+            s.f = [f.contiguous() for f in s.f]
+            s.vel = [v.contiguous() for v in s.vel]
+            assert s.f[0].stride(0) == s.npad and s.vel[0].stride(0) == s.N
+        s.set_sponge(5, 0.6)
+        s.set_drive([0.03, 0.01, 0.0], period=50, ramp=10)
+        s.set_outlet_pressure([0.001])
+        s.run(60, chunk=20)
+        out.append(s.fields())
+    assert np.abs(out[0][1]).max() > 0
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+def test_empty_lattice_keeps_time():
+    """A lattice without fluid advances its clock and drive, alone and beside another in a batch."""
+    empty = lbm.build_lattice(np.ones((4, 4, 4), np.float32), [0, 0, 0], 1.0)
+    s = lbm.Solver(empty, 0.02, model="regularised", block=128)
+    s.set_drive([1.0, 0.5, 0.0], period=8)
+    s.run(3, chunk=2)
+    assert s.tick_value() == 3 and s.drv.item() == pytest.approx(drive(np.array([1.0, 0.5, 0.0]), 8, 0, 2), abs=1e-6)
+    other = lbm.Solver(pipe(), 0.02, model="regularised", block=128)
+    b = batch.BatchSolver([s, other])
+    b.run(5, chunk=2)
+    b.synchronize()
+    assert s.tick_value() == 8 and other.tick_value() == 5
+    assert s.drv.item() == pytest.approx(drive(np.array([1.0, 0.5, 0.0]), 8, 0, 7), abs=1e-6)
