@@ -179,10 +179,14 @@ class Probes:
         with torch.cuda.device(s.dev):
             self.cells = torch.as_tensor(cells if len(cells) else np.zeros(1, np.int32)).to(s.dev)
             self.start = torch.as_tensor(start).to(s.dev)
-            self.psum = torch.zeros(max(1, self.n), dtype=torch.float64, device=s.dev)
-            self.umax = torch.zeros(max(1, self.n), dtype=torch.float32, device=s.dev)
+            # both results in one buffer, so that a sample reads them back in one copy
+            m = max(1, self.n)
+            self._buf = torch.zeros(2 * m, dtype=torch.float64, device=s.dev)
+            self.psum, self.umax = self._buf[:m], self._buf[m:].view(torch.float32)[:m]
+            self._host = torch.empty(2 * m, dtype=torch.float64, pin_memory=True)
 
-    def sample(self):
+    def enqueue(self):
+        """Reduce the fields on the solver's stream and start the read-back; `values` has them once it has passed."""
         s = self.s
         with torch.cuda.device(s.dev), torch.cuda.stream(s.stream):
             check(_lib.load().cs_probe_gather(ctypes_void(s.rho.data_ptr()), ctypes_void(s.vel[s.cur].data_ptr()),
@@ -190,10 +194,18 @@ class Probes:
                                               ctypes_void(self.start.data_ptr()), self.n,
                                               ctypes_void(self.psum.data_ptr()), ctypes_void(self.umax.data_ptr()),
                                               ctypes_void(s.stream.cuda_stream)))
-        s.stream.synchronize()
-        psum = self.psum.cpu().numpy()[:self.n]
-        p = np.where(self.count > 0, psum / np.maximum(self.count, 1), np.nan)
-        return p, float(self.umax.cpu().numpy()[:self.n].max()) if self.n else 0.0
+            self._host.copy_(self._buf, non_blocking=True)
+
+    def values(self):
+        host = self._host.numpy()
+        m = len(host) // 2
+        p = np.where(self.count > 0, host[:self.n] / np.maximum(self.count, 1), np.nan)
+        return p, float(host[m:].view(np.float32)[:self.n].max()) if self.n else 0.0
+
+    def sample(self):
+        self.enqueue()
+        self.s.stream.synchronize()
+        return self.values()
 
 
 def coarse_bins(lat, dx_mm, target_mm=0.1):
@@ -226,7 +238,8 @@ class CoarseMap:
         s = self.s
         with torch.cuda.device(s.dev), torch.cuda.stream(s.stream):
             check(_lib.load().cs_bin_fields(ctypes_void(s.rho.data_ptr()), ctypes_void(s.vel[s.cur].data_ptr()),
-                                            s.vel[s.cur].stride(0), ctypes_void(self.cells.data_ptr()), ctypes_void(self.start.data_ptr()),
+                                            s.vel[s.cur].stride(0), ctypes_void(self.cells.data_ptr()),
+                                            ctypes_void(self.start.data_ptr()),
                                             self.n_bins, ctypes_void(self.p.data_ptr()), ctypes_void(self.u.data_ptr()),
                                             ctypes_void(s.stream.cuda_stream)))
         s.stream.synchronize()
@@ -246,15 +259,27 @@ def run_beats(s, steps_per_beat, beats, every, probes=None, cmap=None, frames=40
     series = {"step": [], "Q": [], "p_open": [], "p_probe": [], "umax": []}
     out = {"t_step": [], "p": [], "u": []}
     total = beats * steps_per_beat
-    coupled = hasattr(s, "Qlast")
+    coupled, deferred = hasattr(s, "Qlast"), hasattr(probes, "enqueue")
+    # a sample's values come back behind the steps on their stream, and the host waits for them once
+    if coupled:
+        q_host = torch.empty_like(s.Qlast.tensor, device="cpu", pin_memory=True)
+        p_host = torch.empty_like(s.p_out, device="cpu", pin_memory=True)
     while s.steps < total:
         s.run(every, chunk=every)
         series["step"].append(s.steps)
         if coupled:
-            series["Q"].append(s.Qlast.numpy().copy())
-            series["p_open"].append(s.p_out.cpu().numpy()[:s.n_open].astype(float))
+            with torch.cuda.device(s.dev), torch.cuda.stream(s.stream):
+                q_host.copy_(s.Qlast.tensor, non_blocking=True)
+                p_host.copy_(s.p_out, non_blocking=True)
+        if deferred:
+            probes.enqueue()
+        if coupled or deferred:
+            s.stream.synchronize()
+        if coupled:
+            series["Q"].append(q_host.numpy().copy())
+            series["p_open"].append(p_host.numpy()[:s.n_open].astype(float))
         if probes is not None:
-            p, um = probes.sample()
+            p, um = probes.values() if deferred else probes.sample()
             series["p_probe"].append(p)
             series["umax"].append(um)
         if s.steps % steps_per_beat == 0:

@@ -92,3 +92,24 @@ def test_empty_lattice_keeps_time():
     b.synchronize()
     assert s.tick_value() == 8 and other.tick_value() == 5
     assert s.drv.item() == pytest.approx(drive(np.array([1.0, 0.5, 0.0]), 8, 0, 7), abs=1e-6)
+
+
+@pytest.mark.parametrize("sizes", [(0, 1, 31), (1023, 1024, 1025), (4095, 4097, 9000)])
+def test_probe_sizes(sizes):
+    """Probes without a cell, below and above a thread's and a block's share, against the fields: the sums in another
+    order of FP64, the largest speed to a float32 square root of three products (4 ulp)."""
+    lat = pipe("open_pipe_R16_L96")
+    s = lbm.Solver(lat, 0.02, model="regularised", order="boundary-first")
+    s.set_drive([0.03])
+    s.run(20)
+    rng = np.random.default_rng(1)
+    idx = [rng.integers(0, s.N, size=n) for n in sizes]
+    probes = simulate.Probes(s, np.concatenate(idx), np.repeat(np.arange(len(sizes)), sizes), len(sizes))
+    p, umax = probes.sample()
+    rho, u = s.rho[s.inv].double().cpu().numpy(), s.fields()[1].astype(np.float64)
+    for k, c in enumerate(idx):
+        if len(c):
+            assert p[k] == pytest.approx(rho[c].mean() / 3, rel=0, abs=1e-12)
+        else:
+            assert np.isnan(p[k])
+    assert umax == pytest.approx(np.linalg.norm(u[np.concatenate(idx)], axis=1).max(), rel=4 * 2.0 ** -23)
