@@ -30,7 +30,6 @@
 
 #include "cs_common.cuh"
 
-#include <utility>
 #include <vector>
 
 namespace cs {
@@ -1040,15 +1039,20 @@ cs_step_desc with_strides(const cs_step_desc& d) {
 constexpr int CARVEOUT = 28;
 
 int set_carveout(const void* fn) {
+    struct Set {
+        int dev;
+        const void* fn;
+    };
     static std::mutex m;
-    static std::vector<std::pair<int, const void*>> done;
+    static Set done[512];               // what has been set; past that the attribute is set again at each call
+    static int n = 0;
     int dev = 0;
     CS_CUDA(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lock(m);
-    const std::pair<int, const void*> key(dev, fn);
-    if (std::find(done.begin(), done.end(), key) != done.end()) return CS_OK;
+    for (int k = 0; k < n; ++k)
+        if (done[k].dev == dev && done[k].fn == fn) return CS_OK;
     CS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, CARVEOUT));
-    done.push_back(key);
+    if (n < 512) done[n++] = Set{dev, fn};
     return CS_OK;
 }
 
