@@ -407,7 +407,10 @@ __device__ __forceinline__ void advance_clock(const cs_step_desc& d, const int a
     }
 }
 
+// Launched programmatically: the first boundary kernel reads its tables while this one works.
 __device__ __forceinline__ void first_clock(const cs_step_desc& d, const int a) {
+    launch_dependents();
+    grid_dependency_wait();
     const float v = drive_value_warp(d, d.tick[a]);
     if (threadIdx.x == 0) d.drive2[a] = v;
 }
@@ -1086,8 +1089,8 @@ int launch_steps(const cs_step_desc* user, int a, int steps, cudaStream_t st) {
         if (rc != CS_OK) return rc;
     }
     if (steps > 0 && grid > 0) {
-        k_clock<<<1, 32, 0, st>>>(*d, a);
-        CS_CHECK_LAUNCH("k_clock");
+        const int rc = launch_pdl(k_clock, dim3(1), dim3(32), st, *d, a);
+        if (rc != CS_OK) return rc;
     }
     for (int s = 0; s < steps; ++s) {
         int rc = CS_OK;
@@ -1426,8 +1429,8 @@ int launch_batch(const cs_batch_desc* b, int a, int steps, cudaStream_t st) {
     for (int i = 0; i < b->n_inst; ++i) empty = empty || b->descs[i].n == 0;
     if (steps > 0)
         for (const BatchGroup& g : gs) {
-            k_clock_batch<<<unsigned(g.n_inst), 32, 0, st>>>(g, a);
-            CS_CHECK_LAUNCH("k_clock_batch");
+            const int rc = launch_batch_pdl(k_clock_batch, unsigned(g.n_inst), 32, st, g, a);
+            if (rc != CS_OK) return rc;
         }
     for (int s = 0; s < steps; ++s) {
         if (empty)
