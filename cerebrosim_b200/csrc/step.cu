@@ -407,10 +407,13 @@ __device__ __forceinline__ void advance_clock(const cs_step_desc& d, const int a
     }
 }
 
-// Launched programmatically: the first boundary kernel reads its tables while this one works.
+// Launched programmatically: the first boundary kernel reads its tables while this one evaluates the drive. Only after
+// the wait, though: what the stream did before this call (a caller's kernel that wrote the tables or the relaxation
+// rates) is then complete, and every later kernel of the call may read them before its own wait. Without boundary links
+// the next kernel is the bulk kernel, which does.
 __device__ __forceinline__ void first_clock(const cs_step_desc& d, const int a) {
-    launch_dependents();
     grid_dependency_wait();
+    launch_dependents();
     const float v = drive_value_warp(d, d.tick[a]);
     if (threadIdx.x == 0) d.drive2[a] = v;
 }
