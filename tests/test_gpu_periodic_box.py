@@ -8,6 +8,7 @@ pytestmark = pytest.mark.gpu
 
 from cerebrosim_b200 import lbm  # noqa: E402
 from oracle import lattice_ref as L  # noqa: E402
+from oracle.step_ref import OracleSolver  # noqa: E402
 
 DIMS = (64, 48, 40)
 PHI = -np.ones(DIMS, np.float32)
@@ -64,3 +65,28 @@ def test_rates_changed_between_calls(model):
     assert np.abs(runs[0][1]).max() > 1e-3
     for p, u in runs[1:]:
         assert np.array_equal(p, runs[0][0]) and np.array_equal(u, runs[0][1])
+
+
+@pytest.mark.parametrize("model", ["regularised", "trt"])
+def test_steps_of_one_call(model):
+    """One call of many steps, each of them launched under the one before, gives the fields of steps that are waited
+    for one by one, bit for bit; both agree with the oracle. Populations of up to 0.006 in magnitude: 61 steps of some
+    thirty roundings, each 2^-24 of that, stay below 7e-7 (a drive one step late would move the velocity by 5e-6)."""
+    lat = lbm.build_lattice(**BOX)
+    f = waves(lat["coords"])
+    one, singles = (start(lbm.Solver(lat, 0.1, model=model), f) for _ in range(2))
+    one.run(61, chunk=200)
+    graph = start(lbm.Solver(lat, 0.1, model=model), f)
+    graph.run(61, chunk=20)
+    for _ in range(61):
+        singles.run(1)
+        singles.synchronize()
+    ref = start(OracleSolver(L.build_lattice(**BOX), 0.1, model=model), f)
+    ref.run(61)
+    p, u = one.fields()
+    for s in (singles, graph):
+        assert np.array_equal(p, s.fields()[0]) and np.array_equal(u, s.fields()[1])
+        assert s.tick_value() == 61 and s.drv.item() == one.drv.item()
+    pr, ur = ref.fields()
+    assert np.abs(ur).max() > 1e-3
+    assert np.abs(p - pr).max() <= 7e-7 and np.abs(u - ur).max() <= 7e-7
