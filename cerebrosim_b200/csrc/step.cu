@@ -2,7 +2,7 @@
 // simulate.k_flux + simulate.k_bc (simulate.py:65-82).
 //
 // One step = two or three kernels on one stream, each launched programmatically so that its blocks start under the last
-// one's (all with one division of the SM's memory: set_carveout), after a one-warp k_clock once per call:
+// one's (all with one division of the SM's memory: set_carveout):
 //  1. k_boundary — the wall / inlet / outlet link list (lbm.py:163-181). One thread per ghost slot (a boundary link of
 //     one direction); it evaluates what the reference's pull produces for that link — Bouzidi interpolation (q < 0.5
 //     with the second node, q >= 0.5 with the node's own population), half-way bounce-back, the velocity inlet with the
@@ -81,6 +81,11 @@ __device__ __forceinline__ float ld_step(Waited w, const float* p) {
     float v;
     if constexpr (FIRST) asm("ld.global.L1::evict_first.f32 %0, [%1];" : "=f"(v) : "l"(p), "r"(w.token));
     else asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p), "r"(w.token));
+    return v;
+}
+__device__ __forceinline__ int32_t ld_step(Waited w, const int32_t* p) {
+    int32_t v;
+    asm("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p), "r"(w.token));
     return v;
 }
 template <bool FIRST>
@@ -405,7 +410,9 @@ __device__ __forceinline__ void store_regularised(void* fout, uint32_t NP, int32
 // ---- 1. boundary-link kernel and clock ----------------------------------------------------------------------------
 // The clock. A step reads its drive, drive2[a], from memory: evaluating it (coefficients from memory, a sine and a
 // cosine per harmonic) took about 4 us on the step's critical path, in the boundary kernel that everything waits for.
-// The bulk kernel of the step before evaluates it beside its nodes, k_clock before the first step of a call.
+// The bulk kernel of the step before evaluates it beside its nodes. Before the first step of a call there is none: its
+// boundary kernel (START) evaluates the drive, each warp for itself, and k_clock where there are no boundary links. (A
+// k_clock of its own before every call was a third launch of calls of one step: 41.4 us against 37.7 without.)
 __device__ __forceinline__ void advance_clock(const cs_step_desc& d, const int a) {
     const int t = d.tick[a];
     const float next = drive_value_warp(d, t + 1);
@@ -416,42 +423,56 @@ __device__ __forceinline__ void advance_clock(const cs_step_desc& d, const int a
     }
 }
 
-// Launched programmatically: the first boundary kernel reads its tables while this one evaluates the drive. Only after
-// the wait, though: what the stream did before this call (a caller's kernel that wrote the tables or the relaxation
-// rates) is then complete, and every later kernel of the call may read them before its own wait. Without boundary links
-// the next kernel is the bulk kernel, which does.
-__device__ __forceinline__ void first_clock(const cs_step_desc& d, const int a) {
+// The first kernel of a call, this or the START boundary kernel, reads nothing and releases nothing before its wait: what
+// the stream did before the call (a caller's kernel that wrote the tables or the relaxation rates) is then complete, and
+// every later kernel of the call may read them before its own wait.
+__global__ void __launch_bounds__(32) k_clock(const cs_step_desc d, const int a) {
     grid_dependency_wait();
     launch_dependents();
     const float v = drive_value_warp(d, d.tick[a]);
     if (threadIdx.x == 0) d.drive2[a] = v;
 }
 
-__global__ void __launch_bounds__(32) k_clock(const cs_step_desc d, const int a) { first_clock(d, a); }
-
 // Without nodes there is no bulk kernel to advance the clock.
 __global__ void __launch_bounds__(32) k_clock_only(const cs_step_desc d, const int a) { advance_clock(d, a); }
 
 // Block (bx, by) of a lattice's boundary-link grid: by = direction, bx = chunk of its ghost slots. Pure latency: the
 // slot's table words (static, read before the previous kernel has ended), its two populations, the ghost's write. Both
-// populations are addressed without a branch, so their loads are in flight together.
-template <int ST>
-__device__ __forceinline__ void boundary_body(const cs_step_desc& d, const int a, const int bx, const int by) {
+// populations are addressed without a branch, so their loads are in flight together. START: the first kernel of a call;
+// publish: this block leaves the drive for the other kernels of the step.
+template <int ST, bool START>
+__device__ __forceinline__ void boundary_body(const cs_step_desc& d, const int a, const int bx, const int by,
+                                              const bool publish) {
     const int i = by;
     const int32_t g = bx * B_THREADS + int(threadIdx.x);
     const uint32_t slot = uint32_t(i) * uint32_t(d.gmax) + uint32_t(g);       // < 27 npad < 2^31
     const bool live = g < d.gmax;
-    const int32_t node = live ? __ldg(d.gnode + slot) : -1;
-    const int32_t info = live ? __ldg(d.ginfo + slot) : 0;
-    const float q = live ? __ldg(d.gq + slot) : 0.0f;
+    Waited t;
+    int32_t node, info;
+    float q, dv = 0.0f;
+    if constexpr (START) {
+        t = grid_dependency_wait();
+        launch_dependents();
+        node = live ? ld_step(t, d.gnode + slot) : -1;
+        info = live ? ld_step(t, d.ginfo + slot) : 0;
+        q = live ? ld_step(t, d.gq + slot) : 0.0f;
+        dv = drive_value_warp(d, d.tick[a]);
+        if (publish && threadIdx.x == 0) d.drive2[a] = dv;
+    } else {
+        node = live ? __ldg(d.gnode + slot) : -1;
+        info = live ? __ldg(d.ginfo + slot) : 0;
+        q = live ? __ldg(d.gq + slot) : 0.0f;
+    }
     const int io = Lat::opp(i);
     const uint32_t NP = uint32_t(d.fstride), own = uint32_t(io) * NP + uint32_t(node);
     // Bouzidi's second population: the wall's second node (q < 0.5) or the node's own along i
     const bool second = info >= 0 && q < 0.5f;
     const uint32_t other = second ? uint32_t(io) * NP + uint32_t(info) : uint32_t(i) * NP + uint32_t(node);
     const float w = weight_rt(i);                                             // the opposite's weight too
-    const Waited t = grid_dependency_wait();
-    launch_dependents();                                    // the bulk kernel may start its static loads
+    if constexpr (!START) {
+        t = grid_dependency_wait();
+        launch_dependents();                                // the bulk kernel may start its static loads
+    }
     if (node < 0) return;                                   // padding slot of a direction with fewer links
     const void* fin = d.f[a];
     const float fo = Pop<ST>::ld(t, fin, own, w);
@@ -472,7 +493,7 @@ __device__ __forceinline__ void boundary_body(const cs_step_desc& d, const int a
         if (info == CS_INLET) {
             // lbm.py:174-177: bounce-back with the prescribed velocity
             const float* u = d.uin + 3 * int64_t(node);
-            const float dv = ld_step(t, d.drive2 + a);
+            if constexpr (!START) dv = ld_step(t, d.drive2 + a);
             const float cu = cx * (__ldg(u) * dv) + cy * (__ldg(u + 1) * dv) + cz * (__ldg(u + 2) * dv);
             v = fo + 6.0f * w * cu;
         } else {
@@ -503,14 +524,14 @@ __device__ __forceinline__ int grid_direction(const int32_t* gblock, int b) {
 
 // Work item `item` of a lattice's boundary-link grid: a 256-slot chunk of one direction (unpadded grid when gblock
 // is set, else ceil(gmax / 256) chunks per direction).
-template <int ST>
+template <int ST, bool START>
 __device__ __forceinline__ void boundary_item(const cs_step_desc& d, const int a, const int item) {
     if (d.gblock[Q] > 0) {
         const int i = grid_direction(d.gblock, item);
-        boundary_body<ST>(d, a, item - d.gblock[i], i);
+        boundary_body<ST, START>(d, a, item - d.gblock[i], i, item == 0);
     } else {
         const int nbx = int(max(int64_t(1), ceil_div(d.gmax, B_THREADS)));
-        boundary_body<ST>(d, a, item % nbx, item / nbx);
+        boundary_body<ST, START>(d, a, item % nbx, item / nbx, item == 0);
     }
 }
 
@@ -520,9 +541,9 @@ __host__ __device__ __forceinline__ int boundary_items(const cs_step_desc& d) {
     return int(Q * nbx);
 }
 
-template <int ST>
+template <int ST, bool START>
 __global__ void __launch_bounds__(B_THREADS) k_boundary(const cs_step_desc d, const int a) {
-    boundary_item<ST>(d, a, blockIdx.x);
+    boundary_item<ST, START>(d, a, blockIdx.x);
 }
 
 // ---- 2. bulk kernel -----------------------------------------------------------------------------------------------
@@ -993,11 +1014,11 @@ StepFn pick_bulk(const cs_step_desc& d) {
     }
 }
 
-StepFn pick_boundary(const cs_step_desc& d) {
+StepFn pick_boundary(const cs_step_desc& d, bool start) {
     switch (d.storage) {
-        case CS_STORE_F16: return k_boundary<CS_STORE_F16>;
-        case CS_STORE_BF16: return k_boundary<CS_STORE_BF16>;
-        default: return k_boundary<CS_STORE_F32>;
+        case CS_STORE_F16: return start ? k_boundary<CS_STORE_F16, true> : k_boundary<CS_STORE_F16, false>;
+        case CS_STORE_BF16: return start ? k_boundary<CS_STORE_BF16, true> : k_boundary<CS_STORE_BF16, false>;
+        default: return start ? k_boundary<CS_STORE_F32, true> : k_boundary<CS_STORE_F32, false>;
     }
 }
 
@@ -1097,12 +1118,12 @@ int launch_steps(const cs_step_desc* user, int a, int steps, cudaStream_t st) {
     const unsigned grid = unsigned(d->n > 0 ? ceil_div(d->n, block) : 0);
     const dim3 bgrid(unsigned(boundary_items(*d)));
     StepFn bulk = pick_bulk(*d);
-    StepFn bound = pick_boundary(*d);
-    for (StepFn fn : {bulk, bound, StepFn(k_bc), StepFn(k_clock)}) {
+    StepFn bound = pick_boundary(*d, false), bound_start = pick_boundary(*d, true);
+    for (StepFn fn : {bulk, bound, bound_start, StepFn(k_bc), StepFn(k_clock)}) {
         const int rc = set_carveout(reinterpret_cast<const void*>(fn));
         if (rc != CS_OK) return rc;
     }
-    if (steps > 0 && grid > 0) {
+    if (steps > 0 && grid > 0 && d->gmax == 0) {
         const int rc = launch_pdl(k_clock, dim3(1), dim3(32), st, *d, a);
         if (rc != CS_OK) return rc;
     }
@@ -1113,7 +1134,7 @@ int launch_steps(const cs_step_desc* user, int a, int steps, cudaStream_t st) {
             k_clock_only<<<1, 32, 0, st>>>(*d, a);
             CS_CHECK_LAUNCH("k_clock_only");
         } else {
-            if (d->gmax > 0) rc = launch_pdl(bound, bgrid, dim3(B_THREADS), st, *d, a);
+            if (d->gmax > 0) rc = launch_pdl(s == 0 ? bound_start : bound, bgrid, dim3(B_THREADS), st, *d, a);
             if (rc != CS_OK) return rc;
             rc = launch_pdl(bulk, dim3(grid + 1), dim3(block), st, *d, a);
             if (rc != CS_OK) return rc;
@@ -1261,13 +1282,13 @@ struct InstanceCursor {
     }
 };
 
-template <int ST>
+template <int ST, bool START>
 __global__ void __launch_bounds__(B_THREADS) k_boundary_batch(const __grid_constant__ BatchGroup g, const int a) {
     const ItemRange r(g.bnd_items);
     InstanceCursor cur(g.bnd_prefix, g.n_inst);
     for (int item = r.lo; item < r.hi; ++item) {
         const int local = cur.next(item);
-        boundary_item<ST>(g.d[cur.inst], a ^ g.parity[cur.inst], local);
+        boundary_item<ST, START>(g.d[cur.inst], a ^ g.parity[cur.inst], local);
     }
     // the previous bulk kernel has finished (boundary_body waited for it) and the next one takes no item before
     // this kernel ends: reset its work counter
@@ -1315,10 +1336,6 @@ __global__ void __launch_bounds__(DENSE_BLOCK, 9) k_bulk_batch_dense(const __gri
     bulk_body<ST, CS_MODEL_REGULARISED, GAL, false, OPEN>(g.d[inst], a ^ g.parity[inst], local, local == 0);
 }
 
-__global__ void __launch_bounds__(32) k_clock_batch(const __grid_constant__ BatchGroup g, const int a) {
-    first_clock(g.d[blockIdx.x], a ^ g.parity[blockIdx.x]);
-}
-
 // The instances without nodes, whose clock no bulk block advances.
 __global__ void __launch_bounds__(32) k_clock_empty_batch(const __grid_constant__ BatchGroup g, const int a) {
     if (g.d[blockIdx.x].n == 0) advance_clock(g.d[blockIdx.x], a ^ g.parity[blockIdx.x]);
@@ -1351,6 +1368,15 @@ BatchFn pick_batch_model(const cs_batch_desc& b, bool dense) {
                      : pick_batch_collision<ST, false, true>(b.model, force, dense);
     return b.gal ? pick_batch_collision<ST, true, false>(b.model, force, dense)
                  : pick_batch_collision<ST, false, false>(b.model, force, dense);
+}
+
+// Also for instances without boundary links: their items are empty, but the first step's evaluate their drive.
+BatchFn pick_batch_boundary(int storage, bool start) {
+    switch (storage) {
+        case CS_STORE_F16: return start ? k_boundary_batch<CS_STORE_F16, true> : k_boundary_batch<CS_STORE_F16, false>;
+        case CS_STORE_BF16: return start ? k_boundary_batch<CS_STORE_BF16, true> : k_boundary_batch<CS_STORE_BF16, false>;
+        default: return start ? k_boundary_batch<CS_STORE_F32, true> : k_boundary_batch<CS_STORE_F32, false>;
+    }
 }
 
 int validate_batch(const cs_batch_desc* b) {
@@ -1432,31 +1458,24 @@ int launch_batch(const cs_batch_desc* b, int a, int steps, cudaStream_t st) {
     BatchFn bulk = b->storage == CS_STORE_F16    ? pick_batch_model<CS_STORE_F16>(*b, dense)
                    : b->storage == CS_STORE_BF16 ? pick_batch_model<CS_STORE_BF16>(*b, dense)
                                                  : pick_batch_model<CS_STORE_F32>(*b, dense);
-    BatchFn bound = b->storage == CS_STORE_F16    ? k_boundary_batch<CS_STORE_F16>
-                    : b->storage == CS_STORE_BF16 ? k_boundary_batch<CS_STORE_BF16>
-                                                  : k_boundary_batch<CS_STORE_F32>;
-    for (BatchFn fn : {bulk, bound, BatchFn(k_bc_batch), BatchFn(k_clock_batch), BatchFn(k_clock_empty_batch)}) {
+    BatchFn bound = pick_batch_boundary(b->storage, false), bound_start = pick_batch_boundary(b->storage, true);
+    for (BatchFn fn : {bulk, bound, bound_start, BatchFn(k_bc_batch), BatchFn(k_clock_empty_batch)}) {
         const int rc = set_carveout(reinterpret_cast<const void*>(fn));
         if (rc != CS_OK) return rc;
     }
     bool empty = false;
     for (int i = 0; i < b->n_inst; ++i) empty = empty || b->descs[i].n == 0;
-    if (steps > 0)
+    for (int s = 0; s < steps; ++s) {
         for (const BatchGroup& g : gs) {
-            const int rc = launch_batch_pdl(k_clock_batch, unsigned(g.n_inst), 32, st, g, a);
+            const unsigned gb = unsigned(b->grid_bnd > 0 ? std::min(b->grid_bnd, g.bnd_items) : g.bnd_items);
+            const int rc = launch_batch_pdl(s == 0 ? bound_start : bound, gb, B_THREADS, st, g, a);
             if (rc != CS_OK) return rc;
         }
-    for (int s = 0; s < steps; ++s) {
         if (empty)
             for (const BatchGroup& g : gs) {
                 k_clock_empty_batch<<<unsigned(g.n_inst), 32, 0, st>>>(g, a);
                 CS_CHECK_LAUNCH("k_clock_empty_batch");
             }
-        for (const BatchGroup& g : gs) {
-            const unsigned gb = unsigned(b->grid_bnd > 0 ? std::min(b->grid_bnd, g.bnd_items) : g.bnd_items);
-            const int rc = launch_batch_pdl(bound, gb, B_THREADS, st, g, a);
-            if (rc != CS_OK) return rc;
-        }
         for (const BatchGroup& g : gs) {
             const unsigned gk = unsigned(b->grid_bulk > 0 ? std::min(b->grid_bulk, g.bulk_items) : g.bulk_items);
             if (gk == 0) continue;

@@ -305,6 +305,8 @@ class Solver:
             self.uin = uin.contiguous()
             self.ghosts = [int(x) for x in ghosts]
             self.gmax = max(self.ghosts) if N else 0
+            # the boundary-link grid without padding blocks, for every step's descriptor
+            self._gblock = (ctypes.c_int32 * (Q + 1))(0, *np.cumsum([-(-g // 256) for g in self.ghosts]).tolist())
             self.npad = N + self.gmax
             gcols = max(1, self.gmax)
             self.links = torch.empty((Q, N), dtype=torch.int32, device=dev)
@@ -433,11 +435,7 @@ class Solver:
     def _desc(self):
         d = _lib.StepDesc()
         d.n, d.npad, d.gmax = self.N, self.npad, self.gmax
-        run = 0
-        for i in range(Q):                       # the boundary-link grid without padding blocks
-            d.gblock[i] = run
-            run += -(-self.ghosts[i] // 256)
-        d.gblock[Q] = run
+        d.gblock = self._gblock
         d.gnode, d.ginfo, d.gq = self.gnode.data_ptr(), self.ginfo.data_ptr(), self.gq.data_ptr()
         d.storage = _lib.STORE[self.storage]
         d.model, d.bouzidi, d.gal = self.model, self.bouzidi, self.gal
