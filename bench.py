@@ -195,11 +195,11 @@ def artery_line(storage, steps, warmup, dev, peak, flush):
                             storage=storage, blocks=(128,), orders=("c", "axis-split", "axis-boundary-first"),
                             steps=100, warmup=30, device=dev, model="regularised")
     s = workloads.make_solver(spec, lat, storage=storage, device=dev, order=best["order"])
-    descs = [s._desc(), s._desc()]
+    descs, layout = [s._desc(), s._desc()], s._layout()
     sp = ctypes.c_void_p(s.stream.cuda_stream)
 
     def step():
-        _lib.check(lib.cs_step(ctypes.byref(descs[s.cur]), s.cur, 1, sp))
+        _lib.check(lib.cs_step_ex(ctypes.byref(descs[s.cur]), ctypes.byref(layout), s.cur, 1, sp))
         s.cur = 1 - s.cur
         s.steps += 1
 
@@ -215,7 +215,7 @@ def artery_line(storage, steps, warmup, dev, peak, flush):
             ev[k][1].record(s.stream)
         b0, b1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         b0.record(s.stream)
-        _lib.check(lib.cs_step(ctypes.byref(descs[s.cur]), s.cur, steps, sp))
+        _lib.check(lib.cs_step_ex(ctypes.byref(descs[s.cur]), ctypes.byref(layout), s.cur, steps, sp))
         b1.record(s.stream)
         s.stream.synchronize()
     if steps % 2:
@@ -448,7 +448,7 @@ def main():
     lib = _lib.load()
     stream = s.stream
     sp = ctypes.c_void_p(stream.cuda_stream)
-    descs = [s._desc(), s._desc()]
+    descs, layout = [s._desc(), s._desc()], s._layout()
     flush_w = torch.empty(FLUSH_BYTES // 4, dtype=torch.float32, device=dev)
     flush_r = torch.ones(FLUSH_BYTES // 4, dtype=torch.float32, device=dev)
     sink = torch.zeros(1, dtype=torch.float32, device=dev)
@@ -460,7 +460,7 @@ def main():
         torch.sum(flush_r, dim=0, keepdim=True, out=sink)
 
     def step(k):
-        _lib.check(lib.cs_step(ctypes.byref(descs[s.cur]), s.cur, 1, sp))
+        _lib.check(lib.cs_step_ex(ctypes.byref(descs[s.cur]), ctypes.byref(layout), s.cur, 1, sp))
         s.cur = 1 - s.cur
         s.steps += 1
 
@@ -488,7 +488,7 @@ def main():
         # the same steps back to back (no flush, one call): the steady state of a run, L2 reuse included
         b0, b1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         b0.record(stream)
-        _lib.check(lib.cs_step(ctypes.byref(descs[s.cur]), s.cur, args.steps, sp))
+        _lib.check(lib.cs_step_ex(ctypes.byref(descs[s.cur]), ctypes.byref(layout), s.cur, args.steps, sp))
         b1.record(stream)
         stream.synchronize()
         if args.steps % 2:

@@ -47,8 +47,11 @@ class StepDesc(ctypes.Structure):
                 ("q_part", ctypes.c_void_p), ("fb_list", ctypes.c_void_p), ("n_fb", ctypes.c_int32),
                 ("q_last", ctypes.c_void_p), ("p_out64", ctypes.c_void_p),
                 ("r_out", ctypes.c_void_p), ("pref", ctypes.c_double), ("alpha", ctypes.c_double),
-                ("gblock", ctypes.c_int32 * 28), ("beat_acc", ctypes.c_void_p), ("drive2", ctypes.c_void_p), ("fstride", ctypes.c_int64),
-                ("vstride", ctypes.c_int64)]
+                ("gblock", ctypes.c_int32 * 28), ("beat_acc", ctypes.c_void_p)]
+
+
+class StepLayout(ctypes.Structure):
+    _fields_ = [("drive2", ctypes.c_void_p), ("fstride", ctypes.c_int64), ("vstride", ctypes.c_int64)]
 
 
 class BatchDesc(ctypes.Structure):
@@ -86,10 +89,15 @@ SIGNATURES = {
     "cs_compress_expand": (_I32, [_P, _P, _P, _I64, _I64, _P, _P]),
     "cs_flux_blocks": (_I32, [_P, _I64, _I64, _I32, _P, _P]),
     "cs_step": (_I32, [ctypes.POINTER(StepDesc), _I32, _I32, _P]),
+    "cs_step_ex": (_I32, [ctypes.POINTER(StepDesc), ctypes.POINTER(StepLayout), _I32, _I32, _P]),
     "cs_step_check": (_I32, [ctypes.POINTER(StepDesc)]),
     "cs_batch_step": (_I32, [ctypes.POINTER(BatchDesc), _I32, _I32, _P]),
+    "cs_batch_step_ex": (_I32, [ctypes.POINTER(BatchDesc), _P, _I32, _I32, _P]),
+    "cs_batch_graph_capture_ex": (_I32, [ctypes.POINTER(BatchDesc), _P, _I32, _I32, _P, ctypes.POINTER(_P)]),
     "cs_batch_graph_capture": (_I32, [ctypes.POINTER(BatchDesc), _I32, _I32, _P, ctypes.POINTER(_P)]),
     "cs_graph_capture": (_I32, [ctypes.POINTER(StepDesc), _I32, _I32, _P, ctypes.POINTER(_P)]),
+    "cs_graph_capture_ex": (_I32, [ctypes.POINTER(StepDesc), ctypes.POINTER(StepLayout), _I32, _I32, _P,
+                                   ctypes.POINTER(_P)]),
     "cs_graph_launch": (_I32, [_P, _P]),
     "cs_graph_destroy": (_I32, [_P]),
     "cs_wss_shear": (_I32, [_P, _I64, _P, _P, _P, _I64, _I32, _D, _P, _P]),
@@ -124,7 +132,7 @@ def load():
         fn.restype = res
         fn.argtypes = args
     if (lib.cs_abi_sizeof(0) != ctypes.sizeof(Opening) or lib.cs_abi_sizeof(1) != ctypes.sizeof(StepDesc)
-            or lib.cs_abi_sizeof(3) != ctypes.sizeof(BatchDesc)):
+            or lib.cs_abi_sizeof(3) != ctypes.sizeof(BatchDesc) or lib.cs_abi_sizeof(4) != ctypes.sizeof(StepLayout)):
         raise ImportError("libcerebrosim_b200.so ABI mismatch: rebuild the library")
     _lib = lib
     return lib

@@ -105,13 +105,14 @@ class BatchSolver:
         """(Re)build the batch descriptor when members or their parameters changed. The instances' descriptors
         are host arrays the library copies into the kernels' parameters at every launch or capture."""
         descs = [m._desc() for m in self.members]
-        raw = b"".join(bytes(d) for d in descs)
+        layouts = [m._layout() for m in self.members]
+        raw = b"".join(bytes(d) for d in descs + layouts)
         key = (raw, tuple(self._parity))
         if key == self._key:
             return
         self._drop_graphs()
         n = len(self.members)
-        self._descs = (_lib.StepDesc * n)(*descs)
+        self._descs, self._layouts = (_lib.StepDesc * n)(*descs), (_lib.StepLayout * n)(*layouts)
         self._par = (ctypes.c_int32 * n)(*self._parity)
         if n > MAX_GROUPS * _lib.BATCH_GROUP:
             raise ValueError(f"{n} instances: at most {MAX_GROUPS * _lib.BATCH_GROUP} per batch")
@@ -162,8 +163,8 @@ class BatchSolver:
                 g = ctypes.c_void_p()
                 self._sync_in()
                 with torch.cuda.device(self.dev), torch.cuda.stream(self.stream):
-                    check(lib.cs_batch_graph_capture(ctypes.byref(self.desc), self.cur, chunk,
-                                                     ctypes_void(self.stream.cuda_stream), ctypes.byref(g)))
+                    check(lib.cs_batch_graph_capture_ex(ctypes.byref(self.desc), self._layouts, self.cur, chunk,
+                                                        ctypes_void(self.stream.cuda_stream), ctypes.byref(g)))
                 self.graphs[key] = g
         else:
             for m in self.members:
@@ -189,12 +190,13 @@ class BatchSolver:
                 key = (self.cur, chunk)
                 if key not in self.graphs:
                     g = ctypes.c_void_p()
-                    check(lib.cs_batch_graph_capture(ctypes.byref(self.desc), self.cur, chunk, sp, ctypes.byref(g)))
+                    check(lib.cs_batch_graph_capture_ex(ctypes.byref(self.desc), self._layouts, self.cur, chunk, sp,
+                                                        ctypes.byref(g)))
                     self.graphs[key] = g
                 for _ in range(full):
                     check(lib.cs_graph_launch(self.graphs[key], sp))
             if rest:
-                check(lib.cs_batch_step(ctypes.byref(self.desc), self.cur, rest, sp))
+                check(lib.cs_batch_step_ex(ctypes.byref(self.desc), self._layouts, self.cur, rest, sp))
                 if rest % 2:
                     self.cur = 1 - self.cur
         self._sync_out()

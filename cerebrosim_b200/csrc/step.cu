@@ -45,6 +45,21 @@ __constant__ int k_cx[Q] = {0, 1, -1, 0, 0, 0, 0, 1, -1, 1, -1, 1, -1, 1, -1, 0,
 __constant__ int k_cy[Q] = {0, 0, 0, 1, -1, 0, 0, 1, -1, -1, 1, 0, 0, 0, 0, 1, -1, 1, -1, 1, -1, 1, -1, -1, 1, 1, -1};
 __constant__ int k_cz[Q] = {0, 0, 0, 0, 0, 1, -1, 0, 0, 0, 0, 1, -1, -1, 1, 1, -1, -1, 1, 1, -1, -1, 1, 1, -1, 1, -1};
 
+// A descriptor with its layout, as the kernels take it.
+struct StepArgs : cs_step_desc {
+    float* drive2;
+    int64_t fstride, vstride;
+    StepArgs() = default;
+    StepArgs(const cs_step_desc& d, const cs_step_layout* l) : cs_step_desc(d) {
+        drive2 = l ? l->drive2 : nullptr;
+        fstride = l && l->fstride ? l->fstride : d.npad;
+        vstride = l && l->vstride ? l->vstride : d.n;
+    }
+    // where the drive of the step that reads buffer a stands (two pointers to choose from by a: the batched FP32 kernels
+    // without a loop spill, 57.2 us against 54.4 a step for four vessels of 100-400 k nodes)
+    __device__ __forceinline__ float* drive_slot(int a) const { return drive2 ? drive2 + a : drive; }
+};
+
 __device__ __forceinline__ float weight_rt(int i) {
     return i == 0 ? 8.0f / 27.0f : (i < 7 ? 2.0f / 27.0f : (i < 19 ? 1.0f / 54.0f : 1.0f / 216.0f));
 }
@@ -151,7 +166,7 @@ template <> struct Pop<CS_STORE_BF16> {
 // ---- helpers ------------------------------------------------------------------------------------------------------
 // drive(t) (lbm.py:95-100, float32) by a whole warp, each lane one term's sine or cosine: a thread alone waits for its
 // coefficients from memory one harmonic after the other (4 us for three).
-__device__ __forceinline__ float drive_value_warp(const cs_step_desc& d, int t) {
+__device__ __forceinline__ float drive_value_warp(const StepArgs& d, int t) {
     const int lane = threadIdx.x & 31;
     const float ph = 2.0f * PI_F * float(t % d.period) / float(d.period);
     float v = d.coef[0];
@@ -196,7 +211,7 @@ __device__ __forceinline__ float ddx_g(int32_t sm, int32_t sp, float gm, float g
 
 // Address of what the difference along link k (1..6) reads for velocity component c: the neighbour's component, or
 // the ghost slot's q.
-__device__ __forceinline__ const float* grad_src(const cs_step_desc& d, const float* vin, int k, int c, int32_t s) {
+__device__ __forceinline__ const float* grad_src(const StepArgs& d, const float* vin, int k, int c, int32_t s) {
     return s < d.n ? vin + int64_t(c) * d.vstride + s : d.gq + int64_t(k) * d.gmax + (s - d.n);
 }
 
@@ -412,36 +427,39 @@ __device__ __forceinline__ void store_regularised(void* fout, uint32_t NP, int32
 // cosine per harmonic) took about 4 us on the step's critical path, in the boundary kernel that everything waits for.
 // The bulk kernel of the step before evaluates it beside its nodes. Before the first step of a call there is none: its
 // boundary kernel (START) evaluates the drive, each warp for itself, and k_clock where there are no boundary links. (A
-// k_clock of its own before every call was a third launch of calls of one step: 41.4 us against 37.7 without.)
-__device__ __forceinline__ void advance_clock(const cs_step_desc& d, const int a) {
+// k_clock of its own before every call was a third launch of calls of one step: 41.4 us against 37.7 without.) A caller
+// without a drive2 has no place for the next step's drive, and every step begins like the first.
+__device__ __forceinline__ void advance_clock(const StepArgs& d, const int a) {
     const int t = d.tick[a];
-    const float next = drive_value_warp(d, t + 1);
-    if ((threadIdx.x & 31) == 0) {
-        *d.drive = d.drive2[a];
-        d.drive2[1 - a] = next;
-        d.tick[1 - a] = t + 1;
+    if (d.drive2) {
+        const float next = drive_value_warp(d, t + 1);
+        if ((threadIdx.x & 31) == 0) {
+            *d.drive = d.drive2[a];
+            d.drive2[1 - a] = next;
+        }
     }
+    if ((threadIdx.x & 31) == 0) d.tick[1 - a] = t + 1;
 }
 
 // The first kernel of a call, this or the START boundary kernel, reads nothing and releases nothing before its wait: what
 // the stream did before the call (a caller's kernel that wrote the tables or the relaxation rates) is then complete, and
 // every later kernel of the call may read them before its own wait.
-__global__ void __launch_bounds__(32) k_clock(const cs_step_desc d, const int a) {
+__global__ void __launch_bounds__(32) k_clock(const StepArgs d, const int a) {
     grid_dependency_wait();
     launch_dependents();
     const float v = drive_value_warp(d, d.tick[a]);
-    if (threadIdx.x == 0) d.drive2[a] = v;
+    if (threadIdx.x == 0) *d.drive_slot(a) = v;
 }
 
 // Without nodes there is no bulk kernel to advance the clock.
-__global__ void __launch_bounds__(32) k_clock_only(const cs_step_desc d, const int a) { advance_clock(d, a); }
+__global__ void __launch_bounds__(32) k_clock_only(const StepArgs d, const int a) { advance_clock(d, a); }
 
 // Block (bx, by) of a lattice's boundary-link grid: by = direction, bx = chunk of its ghost slots. Pure latency: the
 // slot's table words (static, read before the previous kernel has ended), its two populations, the ghost's write. Both
 // populations are addressed without a branch, so their loads are in flight together. START: the first kernel of a call;
 // publish: this block leaves the drive for the other kernels of the step.
 template <int ST, bool START>
-__device__ __forceinline__ void boundary_body(const cs_step_desc& d, const int a, const int bx, const int by,
+__device__ __forceinline__ void boundary_body(const StepArgs& d, const int a, const int bx, const int by,
                                               const bool publish) {
     const int i = by;
     const int32_t g = bx * B_THREADS + int(threadIdx.x);
@@ -457,7 +475,7 @@ __device__ __forceinline__ void boundary_body(const cs_step_desc& d, const int a
         info = live ? ld_step(t, d.ginfo + slot) : 0;
         q = live ? ld_step(t, d.gq + slot) : 0.0f;
         dv = drive_value_warp(d, d.tick[a]);
-        if (publish && threadIdx.x == 0) d.drive2[a] = dv;
+        if (publish && threadIdx.x == 0) *d.drive_slot(a) = dv;
     } else {
         node = live ? __ldg(d.gnode + slot) : -1;
         info = live ? __ldg(d.ginfo + slot) : 0;
@@ -493,7 +511,7 @@ __device__ __forceinline__ void boundary_body(const cs_step_desc& d, const int a
         if (info == CS_INLET) {
             // lbm.py:174-177: bounce-back with the prescribed velocity
             const float* u = d.uin + 3 * int64_t(node);
-            if constexpr (!START) dv = ld_step(t, d.drive2 + a);
+            if constexpr (!START) dv = ld_step(t, d.drive_slot(a));
             const float cu = cx * (__ldg(u) * dv) + cy * (__ldg(u + 1) * dv) + cz * (__ldg(u + 2) * dv);
             v = fo + 6.0f * w * cu;
         } else {
@@ -525,7 +543,7 @@ __device__ __forceinline__ int grid_direction(const int32_t* gblock, int b) {
 // Work item `item` of a lattice's boundary-link grid: a 256-slot chunk of one direction (unpadded grid when gblock
 // is set, else ceil(gmax / 256) chunks per direction).
 template <int ST, bool START>
-__device__ __forceinline__ void boundary_item(const cs_step_desc& d, const int a, const int item) {
+__device__ __forceinline__ void boundary_item(const StepArgs& d, const int a, const int item) {
     if (d.gblock[Q] > 0) {
         const int i = grid_direction(d.gblock, item);
         boundary_body<ST, START>(d, a, item - d.gblock[i], i, item == 0);
@@ -542,7 +560,7 @@ __host__ __device__ __forceinline__ int boundary_items(const cs_step_desc& d) {
 }
 
 template <int ST, bool START>
-__global__ void __launch_bounds__(B_THREADS) k_boundary(const cs_step_desc d, const int a) {
+__global__ void __launch_bounds__(B_THREADS) k_boundary(const StepArgs d, const int a) {
     boundary_item<ST, START>(d, a, blockIdx.x);
 }
 
@@ -564,7 +582,7 @@ __device__ __forceinline__ void store_pairs(void* fout, uint32_t NP, int32_t n, 
 }
 
 template <int ST, int MODEL, bool GAL, bool FORCE, bool FIRST>
-__device__ __forceinline__ void node_update(const cs_step_desc& d, int a, int32_t n, float& ux_o, float& uy_o,
+__device__ __forceinline__ void node_update(const StepArgs& d, int a, int32_t n, float& ux_o, float& uy_o,
                                             float& uz_o) {
     const int32_t N = int32_t(d.n), NV = int32_t(d.vstride);
     const uint32_t NP = uint32_t(d.fstride);
@@ -593,7 +611,7 @@ __device__ __forceinline__ void node_update(const cs_step_desc& d, int a, int32_
     }
     const float om_signed = __ldg(d.om + n);
     const Waited waited = grid_dependency_wait();
-    const float dv = ld_step(waited, d.drive2 + a);
+    const float dv = ld_step(waited, d.drive_slot(a));
     const float upx = ld_step(waited, vin + n), upy = ld_step(waited, vin + NV + n),
                 upz = ld_step(waited, vin + 2 * NV + n);
 
@@ -808,7 +826,7 @@ __device__ __forceinline__ void node_update(const cs_step_desc& d, int a, int32_
 // OPEN: the lattice may have open ends (n_open > 0); compiled apart for the kernels that lose by carrying their
 // reduction. clock: this block also advances the clock.
 template <int ST, int MODEL, bool GAL, bool FORCE, bool OPEN, bool FIRST = false>
-__device__ __forceinline__ void bulk_body(const cs_step_desc& d, const int a, const int bx, const bool clock) {
+__device__ __forceinline__ void bulk_body(const StepArgs& d, const int a, const int bx, const bool clock) {
     const int32_t n0 = int32_t(bx) * int32_t(blockDim.x);
     const int32_t n = n0 + int32_t(threadIdx.x);
     // read after the update: bring the line in meanwhile, at the cost of no register
@@ -869,7 +887,7 @@ __device__ __forceinline__ void bulk_body(const cs_step_desc& d, const int a, co
 
 // A block of a single lattice's grid; the first is the clock, beside the node blocks.
 template <int ST, int MODEL, bool GAL, bool FORCE, bool OPEN, bool FIRST = false>
-__device__ __forceinline__ void bulk_block(const cs_step_desc& d, const int a) {
+__device__ __forceinline__ void bulk_block(const StepArgs& d, const int a) {
     if (blockIdx.x == 0) {
         grid_dependency_wait();
         if (threadIdx.x < 32) advance_clock(d, a);
@@ -880,7 +898,7 @@ __device__ __forceinline__ void bulk_block(const cs_step_desc& d, const int a) {
 }
 
 template <int ST, int MODEL, bool GAL, bool FORCE, bool OPEN>
-__global__ void __launch_bounds__(MAX_BLOCK, MIN_BLOCKS) k_bulk(const cs_step_desc d, const int a) {
+__global__ void __launch_bounds__(MAX_BLOCK, MIN_BLOCKS) k_bulk(const StepArgs d, const int a) {
     bulk_block<ST, MODEL, GAL, FORCE, OPEN>(d, a);
 }
 
@@ -899,7 +917,7 @@ constexpr int DENSE_BLOCK = 128;
 constexpr int dense_blocks(int st) { return st == CS_STORE_F32 ? 8 : 9; }
 
 template <int ST, bool GAL, bool FIRST>
-__global__ void __launch_bounds__(DENSE_BLOCK, dense_blocks(ST)) k_bulk_dense(const cs_step_desc d, const int a) {
+__global__ void __launch_bounds__(DENSE_BLOCK, dense_blocks(ST)) k_bulk_dense(const StepArgs d, const int a) {
     bulk_block<ST, CS_MODEL_REGULARISED, GAL, false, true, FIRST>(d, a);
 }
 
@@ -912,7 +930,7 @@ constexpr int BC_THREADS = 512;
 // latency on the path from one step to the next: launched programmatically, it reads fb_list before the bulk kernel has
 // ended and lets the next boundary kernel become resident while it works. A tree over all threads per open end and an
 // ordinary launch took 8.3 us on 1487 rows, a quarter of a step of 190 k nodes.
-__device__ __forceinline__ void bc_body(const cs_step_desc& d) {
+__device__ __forceinline__ void bc_body(const StepArgs& d) {
     __shared__ double s_w[BC_THREADS / 32][MAX_OPEN];
     constexpr int AHEAD = 4;
     launch_dependents();
@@ -973,9 +991,9 @@ __device__ __forceinline__ void bc_body(const cs_step_desc& d) {
     }
 }
 
-__global__ void __launch_bounds__(BC_THREADS) k_bc(const cs_step_desc d, const int) { bc_body(d); }
+__global__ void __launch_bounds__(BC_THREADS) k_bc(const StepArgs d, const int) { bc_body(d); }
 
-using StepFn = void (*)(const cs_step_desc, const int);
+using StepFn = void (*)(const StepArgs, const int);
 
 template <int ST, bool GAL, bool OPEN>
 StepFn pick_collision(int model, bool force, int block, bool first) {
@@ -995,7 +1013,7 @@ int64_t l2_bytes() {
 }
 
 template <int ST>
-StepFn pick_model(const cs_step_desc& d) {
+StepFn pick_model(const StepArgs& d) {
     const bool force = d.force[0] != 0.0f || d.force[1] != 0.0f || d.force[2] != 0.0f;
     const int block = d.block ? d.block : MAX_BLOCK;
     const bool first = 2 * int64_t(Q) * d.fstride * (ST == CS_STORE_F32 ? 4 : 2) <= l2_bytes();
@@ -1006,7 +1024,7 @@ StepFn pick_model(const cs_step_desc& d) {
                  : pick_collision<ST, false, false>(d.model, force, block, first);
 }
 
-StepFn pick_bulk(const cs_step_desc& d) {
+StepFn pick_bulk(const StepArgs& d) {
     switch (d.storage) {
         case CS_STORE_F16: return pick_model<CS_STORE_F16>(d);
         case CS_STORE_BF16: return pick_model<CS_STORE_BF16>(d);
@@ -1014,7 +1032,7 @@ StepFn pick_bulk(const cs_step_desc& d) {
     }
 }
 
-StepFn pick_boundary(const cs_step_desc& d, bool start) {
+StepFn pick_boundary(const StepArgs& d, bool start) {
     switch (d.storage) {
         case CS_STORE_F16: return start ? k_boundary<CS_STORE_F16, true> : k_boundary<CS_STORE_F16, false>;
         case CS_STORE_BF16: return start ? k_boundary<CS_STORE_BF16, true> : k_boundary<CS_STORE_BF16, false>;
@@ -1022,19 +1040,16 @@ StepFn pick_boundary(const cs_step_desc& d, bool start) {
     }
 }
 
-cs_step_desc with_strides(const cs_step_desc& d);
-
-int validate(const cs_step_desc* user) {
-    if (!user) return fail(CS_ERR_ARG, "cs_step: null descriptor");
-    const cs_step_desc filled = with_strides(*user);
-    const cs_step_desc* d = &filled;
+int validate(const cs_step_desc* d, const cs_step_layout* layout) {
+    if (!d) return fail(CS_ERR_ARG, "cs_step: null descriptor");
     if (d->n < 0 || d->n >= (int64_t(1) << 30)) return fail(CS_ERR_SIZE, "cs_step: n = %lld", (long long)d->n);
     if (d->gmax < 0 || d->npad != d->n + d->gmax || int64_t(Q) * d->npad >= (int64_t(1) << 31))
         return fail(CS_ERR_SIZE, "cs_step: npad %lld must be n + gmax with 27 * npad < 2^31", (long long)d->npad);
-    if (d->fstride < d->npad || int64_t(Q) * d->fstride >= (int64_t(1) << 31) || d->vstride < d->n ||
-        3 * d->vstride >= (int64_t(1) << 31))
+    const int64_t fstride = layout && layout->fstride ? layout->fstride : d->npad;
+    const int64_t vstride = layout && layout->vstride ? layout->vstride : d->n;
+    if (fstride < d->npad || fstride > INT32_MAX / Q || vstride < d->n || vstride > INT32_MAX / 3)
         return fail(CS_ERR_SIZE, "cs_step: row strides %lld (npad %lld; 27 rows below 2^31) and %lld (n %lld)",
-                    (long long)d->fstride, (long long)d->npad, (long long)d->vstride, (long long)d->n);
+                    (long long)fstride, (long long)d->npad, (long long)vstride, (long long)d->n);
     if (d->gblock[0] != 0) return fail(CS_ERR_ARG, "cs_step: gblock[0] = %d", d->gblock[0]);
     for (int i = 0; i < Q; ++i) {
         const int64_t w = int64_t(d->gblock[i + 1]) - d->gblock[i];
@@ -1047,7 +1062,7 @@ int validate(const cs_step_desc* user) {
     if (d->block != 0 && (d->block < 32 || d->block > MAX_BLOCK || d->block % 32))
         return fail(CS_ERR_ARG, "cs_step: block %d (32..%d, multiple of 32)", d->block, MAX_BLOCK);
     if (d->period < 1 || d->nh < 0 || d->ramp < 0) return fail(CS_ERR_ARG, "cs_step: period %d nh %d ramp %d", d->period, d->nh, d->ramp);
-    if (!d->tick || !d->drive || !d->drive2 || !d->coef || !d->p_out || d->n_out < 1)
+    if (!d->tick || !d->drive || !d->coef || !d->p_out || d->n_out < 1)
         return fail(CS_ERR_ARG, "cs_step: null clock / outlet state");
     if (d->n > 0 && (!d->f[0] || !d->f[1] || !d->vel[0] || !d->vel[1] || !d->rho || !d->lcode || !d->uin || !d->om))
         return fail(CS_ERR_ARG, "cs_step: null lattice buffer");
@@ -1059,14 +1074,6 @@ int validate(const cs_step_desc* user) {
                           (d->n_flux > 0 && (!d->flux_idx || !d->flux_w || !d->flux_slot))))
         return fail(CS_ERR_ARG, "cs_step: null flux buffer");
     return CS_OK;
-}
-
-// A descriptor with its row strides filled in (0: rows back to back).
-cs_step_desc with_strides(const cs_step_desc& d) {
-    cs_step_desc r = d;
-    if (r.fstride == 0) r.fstride = r.npad;
-    if (r.vstride == 0) r.vstride = r.n;
-    return r;
 }
 
 // One division of the SM's memory between L1 and shared memory for every kernel of a step. By default the driver picks
@@ -1095,7 +1102,7 @@ int set_carveout(const void* fn) {
 }
 
 // Launch with programmatic stream serialization, so the kernel's static prologue overlaps the previous kernel.
-int launch_pdl(StepFn fn, dim3 grid, dim3 block, cudaStream_t st, const cs_step_desc& d, int a) {
+int launch_pdl(StepFn fn, dim3 grid, dim3 block, cudaStream_t st, const StepArgs& d, int a) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -1111,9 +1118,8 @@ int launch_pdl(StepFn fn, dim3 grid, dim3 block, cudaStream_t st, const cs_step_
     return CS_OK;
 }
 
-int launch_steps(const cs_step_desc* user, int a, int steps, cudaStream_t st) {
-    const cs_step_desc filled = with_strides(*user);
-    const cs_step_desc* d = &filled;
+int launch_steps(const StepArgs& args, int a, int steps, cudaStream_t st) {
+    const StepArgs* d = &args;
     const int block = d->block ? d->block : MAX_BLOCK;
     const unsigned grid = unsigned(d->n > 0 ? ceil_div(d->n, block) : 0);
     const dim3 bgrid(unsigned(boundary_items(*d)));
@@ -1123,18 +1129,16 @@ int launch_steps(const cs_step_desc* user, int a, int steps, cudaStream_t st) {
         const int rc = set_carveout(reinterpret_cast<const void*>(fn));
         if (rc != CS_OK) return rc;
     }
-    if (steps > 0 && grid > 0 && d->gmax == 0) {
-        const int rc = launch_pdl(k_clock, dim3(1), dim3(32), st, *d, a);
-        if (rc != CS_OK) return rc;
-    }
     for (int s = 0; s < steps; ++s) {
+        const bool start = s == 0 || !d->drive2;
         int rc = CS_OK;
         if (grid == 0) {
             k_clock<<<1, 32, 0, st>>>(*d, a);
             k_clock_only<<<1, 32, 0, st>>>(*d, a);
             CS_CHECK_LAUNCH("k_clock_only");
         } else {
-            if (d->gmax > 0) rc = launch_pdl(s == 0 ? bound_start : bound, bgrid, dim3(B_THREADS), st, *d, a);
+            if (d->gmax > 0) rc = launch_pdl(start ? bound_start : bound, bgrid, dim3(B_THREADS), st, *d, a);
+            else if (start) rc = launch_pdl(k_clock, dim3(1), dim3(32), st, *d, a);
             if (rc != CS_OK) return rc;
             rc = launch_pdl(bulk, dim3(grid + 1), dim3(block), st, *d, a);
             if (rc != CS_OK) return rc;
@@ -1176,11 +1180,15 @@ extern "C" int cs_flux_blocks(const int32_t* flux_idx, int64_t n_flux, int64_t n
     return CS_OK;
 }
 
-extern "C" int cs_step(const cs_step_desc* d, int32_t a, int32_t steps, void* stream) {
-    int rc = validate(d);
+extern "C" int cs_step_ex(const cs_step_desc* d, const cs_step_layout* layout, int32_t a, int32_t steps, void* stream) {
+    int rc = validate(d, layout);
     if (rc != CS_OK) return rc;
     if ((a != 0 && a != 1) || steps < 0) return fail(CS_ERR_ARG, "cs_step: a %d steps %d", a, steps);
-    return launch_steps(d, a, steps, as_stream(stream));
+    return launch_steps(StepArgs(*d, layout), a, steps, as_stream(stream));
+}
+
+extern "C" int cs_step(const cs_step_desc* d, int32_t a, int32_t steps, void* stream) {
+    return cs_step_ex(d, nullptr, a, steps, stream);
 }
 
 namespace {
@@ -1189,14 +1197,15 @@ struct Graph {
 };
 }  // namespace
 
-extern "C" int cs_graph_capture(const cs_step_desc* d, int32_t a, int32_t steps, void* stream, void** graph) {
-    int rc = validate(d);
+extern "C" int cs_graph_capture_ex(const cs_step_desc* d, const cs_step_layout* layout, int32_t a, int32_t steps,
+                                   void* stream, void** graph) {
+    int rc = validate(d, layout);
     if (rc != CS_OK) return rc;
     if ((a != 0 && a != 1) || steps < 1 || !graph) return fail(CS_ERR_ARG, "cs_graph_capture: a %d steps %d", a, steps);
     cudaStream_t st = as_stream(stream);
     if (st == nullptr) return fail(CS_ERR_ARG, "cs_graph_capture: the legacy default stream cannot be captured");
     CS_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    rc = launch_steps(d, a, steps, st);
+    rc = launch_steps(StepArgs(*d, layout), a, steps, st);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(st, &g);
     if (rc != CS_OK) {
@@ -1210,6 +1219,10 @@ extern "C" int cs_graph_capture(const cs_step_desc* d, int32_t a, int32_t steps,
     if (e != cudaSuccess) return fail(CS_ERR_CUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(e));
     *graph = new Graph{ex};
     return CS_OK;
+}
+
+extern "C" int cs_graph_capture(const cs_step_desc* d, int32_t a, int32_t steps, void* stream, void** graph) {
+    return cs_graph_capture_ex(d, nullptr, a, steps, stream, graph);
 }
 
 extern "C" int cs_graph_launch(void* graph, void* stream) {
@@ -1227,7 +1240,7 @@ extern "C" int cs_graph_destroy(void* graph) {
     return CS_OK;
 }
 
-extern "C" int cs_step_check(const cs_step_desc* d) { return validate(d); }
+extern "C" int cs_step_check(const cs_step_desc* d) { return validate(d, nullptr); }
 
 // ---- batched step -------------------------------------------------------------------------------------------------
 // The instances' descriptors travel in the kernels' parameter space (constant bank), CS_BATCH_GROUP instances per
@@ -1242,7 +1255,7 @@ struct BatchGroup {
     int32_t bulk_prefix[CS_BATCH_GROUP + 1];
     int32_t bnd_prefix[CS_BATCH_GROUP + 1];
     int32_t parity[CS_BATCH_GROUP];
-    cs_step_desc d[CS_BATCH_GROUP];
+    StepArgs d[CS_BATCH_GROUP];
 };
 static_assert(sizeof(BatchGroup) < 32000, "batched kernel parameters exceed the 32 KB limit");
 
@@ -1342,7 +1355,7 @@ __global__ void __launch_bounds__(32) k_clock_empty_batch(const __grid_constant_
 }
 
 __global__ void __launch_bounds__(BC_THREADS) k_bc_batch(const __grid_constant__ BatchGroup g, const int) {
-    const cs_step_desc& d = g.d[blockIdx.x];
+    const StepArgs& d = g.d[blockIdx.x];
     if (d.n_open > 0) {
         bc_body(d);
     } else {
@@ -1379,7 +1392,7 @@ BatchFn pick_batch_boundary(int storage, bool start) {
     }
 }
 
-int validate_batch(const cs_batch_desc* b) {
+int validate_batch(const cs_batch_desc* b, const cs_step_layout* layouts) {
     if (!b) return fail(CS_ERR_ARG, "cs_batch_step: null descriptor");
     if (b->n_inst < 1 || !b->descs || !b->parity || !b->counter)
         return fail(CS_ERR_ARG, "cs_batch_step: %d instances or null tables", b->n_inst);
@@ -1392,7 +1405,7 @@ int validate_batch(const cs_batch_desc* b) {
     int64_t items = 0;
     for (int i = 0; i < b->n_inst; ++i) {
         const cs_step_desc& d = b->descs[i];
-        const int rc = validate(&d);
+        const int rc = validate(&d, layouts ? layouts + i : nullptr);
         if (rc != CS_OK) return rc;
         if (d.storage != b->storage || d.model != b->model || d.gal != b->gal || d.block != b->block)
             return fail(CS_ERR_ARG, "cs_batch_step: instance %d differs from the batch in storage, model, Galilean "
@@ -1411,7 +1424,7 @@ int validate_batch(const cs_batch_desc* b) {
 }
 
 // The launch groups of a batch: CS_BATCH_GROUP instances each, work items counted per instance.
-std::vector<BatchGroup> make_groups(const cs_batch_desc* b) {
+std::vector<BatchGroup> make_groups(const cs_batch_desc* b, const cs_step_layout* layouts) {
     std::vector<BatchGroup> gs;
     for (int i0 = 0; i0 < b->n_inst; i0 += CS_BATCH_GROUP) {
         BatchGroup g;
@@ -1420,7 +1433,7 @@ std::vector<BatchGroup> make_groups(const cs_batch_desc* b) {
         g.counter = b->counter + i0 / CS_BATCH_GROUP;
         int64_t bulk = 0, bnd = 0;
         for (int k = 0; k < g.n_inst; ++k) {
-            const cs_step_desc d = with_strides(b->descs[i0 + k]);
+            const StepArgs d(b->descs[i0 + k], layouts ? layouts + i0 + k : nullptr);
             g.d[k] = d;
             g.parity[k] = b->parity[i0 + k];
             g.bulk_prefix[k] = int32_t(bulk);
@@ -1452,8 +1465,8 @@ int launch_batch_pdl(BatchFn fn, unsigned grid, unsigned block, cudaStream_t st,
     return CS_OK;
 }
 
-int launch_batch(const cs_batch_desc* b, int a, int steps, cudaStream_t st) {
-    const std::vector<BatchGroup> gs = make_groups(b);
+int launch_batch(const cs_batch_desc* b, const cs_step_layout* layouts, int a, int steps, cudaStream_t st) {
+    const std::vector<BatchGroup> gs = make_groups(b, layouts);
     const bool dense = b->grid_bulk == 0 && b->block <= DENSE_BLOCK;     // one block per item: k_bulk_batch_dense
     BatchFn bulk = b->storage == CS_STORE_F16    ? pick_batch_model<CS_STORE_F16>(*b, dense)
                    : b->storage == CS_STORE_BF16 ? pick_batch_model<CS_STORE_BF16>(*b, dense)
@@ -1463,12 +1476,15 @@ int launch_batch(const cs_batch_desc* b, int a, int steps, cudaStream_t st) {
         const int rc = set_carveout(reinterpret_cast<const void*>(fn));
         if (rc != CS_OK) return rc;
     }
-    bool empty = false;
-    for (int i = 0; i < b->n_inst; ++i) empty = empty || b->descs[i].n == 0;
+    bool empty = false, every = !layouts;           // every: some instance has no place for the next step's drive
+    for (int i = 0; i < b->n_inst; ++i) {
+        empty = empty || b->descs[i].n == 0;
+        every = every || !layouts[i].drive2;
+    }
     for (int s = 0; s < steps; ++s) {
         for (const BatchGroup& g : gs) {
             const unsigned gb = unsigned(b->grid_bnd > 0 ? std::min(b->grid_bnd, g.bnd_items) : g.bnd_items);
-            const int rc = launch_batch_pdl(s == 0 ? bound_start : bound, gb, B_THREADS, st, g, a);
+            const int rc = launch_batch_pdl(s == 0 || every ? bound_start : bound, gb, B_THREADS, st, g, a);
             if (rc != CS_OK) return rc;
         }
         if (empty)
@@ -1496,22 +1512,28 @@ int launch_batch(const cs_batch_desc* b, int a, int steps, cudaStream_t st) {
 }  // namespace
 }  // namespace cs
 
-extern "C" int cs_batch_step(const cs_batch_desc* b, int32_t a, int32_t steps, void* stream) {
-    int rc = validate_batch(b);
+extern "C" int cs_batch_step_ex(const cs_batch_desc* b, const cs_step_layout* layouts, int32_t a, int32_t steps,
+                                void* stream) {
+    int rc = validate_batch(b, layouts);
     if (rc != CS_OK) return rc;
     if ((a != 0 && a != 1) || steps < 0) return fail(CS_ERR_ARG, "cs_batch_step: a %d steps %d", a, steps);
-    return launch_batch(b, a, steps, as_stream(stream));
+    return launch_batch(b, layouts, a, steps, as_stream(stream));
 }
 
-extern "C" int cs_batch_graph_capture(const cs_batch_desc* b, int32_t a, int32_t steps, void* stream, void** graph) {
-    int rc = validate_batch(b);
+extern "C" int cs_batch_step(const cs_batch_desc* b, int32_t a, int32_t steps, void* stream) {
+    return cs_batch_step_ex(b, nullptr, a, steps, stream);
+}
+
+extern "C" int cs_batch_graph_capture_ex(const cs_batch_desc* b, const cs_step_layout* layouts, int32_t a, int32_t steps,
+                                         void* stream, void** graph) {
+    int rc = validate_batch(b, layouts);
     if (rc != CS_OK) return rc;
     if ((a != 0 && a != 1) || steps < 1 || !graph)
         return fail(CS_ERR_ARG, "cs_batch_graph_capture: a %d steps %d", a, steps);
     cudaStream_t st = as_stream(stream);
     if (st == nullptr) return fail(CS_ERR_ARG, "cs_batch_graph_capture: the legacy default stream cannot be captured");
     CS_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    rc = launch_batch(b, a, steps, st);
+    rc = launch_batch(b, layouts, a, steps, st);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(st, &g);
     if (rc != CS_OK) {
@@ -1525,4 +1547,8 @@ extern "C" int cs_batch_graph_capture(const cs_batch_desc* b, int32_t a, int32_t
     if (e != cudaSuccess) return fail(CS_ERR_CUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(e));
     *graph = new Graph{ex};
     return CS_OK;
+}
+
+extern "C" int cs_batch_graph_capture(const cs_batch_desc* b, int32_t a, int32_t steps, void* stream, void** graph) {
+    return cs_batch_graph_capture_ex(b, nullptr, a, steps, stream, graph);
 }

@@ -452,10 +452,12 @@ class Solver:
         d.tick, d.drive, d.coef = self.tick.data_ptr(), self.drv.data_ptr(), self.coef.data_ptr()
         d.nh, d.period, d.ramp = self.nh, self.period, self.ramp
         d.p_out64 = self.p_out64.data_ptr()
-        d.drive2 = self._drv2.data_ptr()
-        d.fstride, d.vstride = self.f[0].stride(0), self.vel[0].stride(0)
         self._fill_desc(d)
         return d
+
+    def _layout(self):
+        """What the step takes beside the descriptor: the drive's two slots and the buffers' row strides."""
+        return _lib.StepLayout(self._drv2.data_ptr(), self.f[0].stride(0), self.vel[0].stride(0))
 
     def _fill_desc(self, d):
         """Hook for subclasses that add the outlet-resistance coupling."""
@@ -463,7 +465,8 @@ class Solver:
 
     def _launch(self, a):
         """One step reading buffer a and writing 1 - a (lbm.py:422-428)."""
-        check(_lib.load().cs_step(ctypes.byref(self._desc()), int(a), 1, ctypes_void(self.stream.cuda_stream)))
+        check(_lib.load().cs_step_ex(ctypes.byref(self._desc()), ctypes.byref(self._layout()), int(a), 1,
+                                     ctypes_void(self.stream.cuda_stream)))
 
     def _drop_graphs(self):
         lib = _lib.load()
@@ -476,8 +479,8 @@ class Solver:
     def _capture(self, a, chunk):
         if type(self)._launch is Solver._launch:
             g = ctypes.c_void_p()
-            check(_lib.load().cs_graph_capture(ctypes.byref(self._desc()), int(a), int(chunk),
-                                               ctypes_void(self.stream.cuda_stream), ctypes.byref(g)))
+            check(_lib.load().cs_graph_capture_ex(ctypes.byref(self._desc()), ctypes.byref(self._layout()), int(a),
+                                                  int(chunk), ctypes_void(self.stream.cuda_stream), ctypes.byref(g)))
             return g
         # a subclass extended _launch: capture its Python-level launches with torch's graph API
         graph = torch.cuda.CUDAGraph()
@@ -519,8 +522,8 @@ class Solver:
                     self._replay(self.graphs[key])
             if rest and type(self)._launch is Solver._launch:
                 # the leftover steps in one library call (the same launches, without a descriptor per step)
-                check(_lib.load().cs_step(ctypes.byref(self._desc()), int(self.cur), int(rest),
-                                          ctypes_void(self.stream.cuda_stream)))
+                check(_lib.load().cs_step_ex(ctypes.byref(self._desc()), ctypes.byref(self._layout()), int(self.cur),
+                                             int(rest), ctypes_void(self.stream.cuda_stream)))
                 self.cur ^= rest & 1
             else:
                 for _ in range(rest):

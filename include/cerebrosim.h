@@ -183,8 +183,8 @@ typedef struct cs_step_desc {
     float magic;             /* TRT magic parameter */
     float force[3];          /* body force, scaled by the drive */
     int32_t block;           /* threads per block of the bulk kernel; 0 = default */
-    void* f[2];              /* populations (27 rows of npad, fstride apart) in `storage` format, link-major */
-    float* vel[2];           /* velocity, SoA: vel[b][c * vstride + node] */
+    void* f[2];              /* populations (27 * npad) in `storage` format, link-major */
+    float* vel[2];           /* velocity, SoA: vel[b][c * n + node] */
     float* rho;              /* density deviation (n) */
     const int32_t* lcode;    /* compressed connectivity (n) from cs_compress_fill */
     const int32_t* segdelta; /* (CS_SEG_STRIDE * n_seg), 16-byte aligned */
@@ -223,12 +223,16 @@ typedef struct cs_step_desc {
      * beat_acc[k] and q_last[k] to beat_acc[n_open + k] (FP64) and 1 to beat_acc[2 * n_open]; the caller zeroes
      * it at a beat's start and divides by the count at its end (the beat means of simulate.py:325-333). */
     double* beat_acc;
-    float* drive2;           /* (2): the drive of the step that reads buffer a, written by the step before it, and for
-                              * the first step of a call by a one-warp kernel */
+} cs_step_desc;
+
+/* What the _ex entry points take beside a descriptor (null, or any field zero: as the entry points without it). */
+typedef struct cs_step_layout {
+    float* drive2;           /* DEVICE (2): the drive of the step that reads buffer a, written by the step before it.
+                              * Without it every step evaluates its drive before anything else */
     int64_t fstride;         /* elements between population rows, >= npad, 27 * fstride < 2^31; 0: npad. Rows that start
                               * on a 128-byte line cost the kernel's stores no split sectors */
-    int64_t vstride;         /* elements between velocity rows, >= n; 0: n */
-} cs_step_desc;
+    int64_t vstride;         /* elements between velocity rows, >= n, 3 * vstride < 2^31; 0: n */
+} cs_step_layout;
 
 /* Block partition of a sorted flux list for `block` threads per block: out[b] = first entry with
  * flux_idx >= b * block, b = 0 .. ceil(n / block). */
@@ -236,9 +240,11 @@ int cs_flux_blocks(const int32_t* flux_idx, int64_t n_flux, int64_t n, int32_t b
 
 /* Enqueue `steps` steps, the first reading buffer a (0/1) and writing 1 - a, alternating (lbm.py:422-428). A step
  * is the boundary-link kernel (one block per 256 boundary links of a direction; none without any), the bulk kernel
- * (its first block advances the clock and evaluates the next step's drive) and, when n_open > 0, the one-block k_bc
- * kernel; a one-warp kernel evaluates the drive of the call's first step before them. */
+ * (its first block advances the clock and, given drive2, evaluates the next step's drive) and, when n_open > 0, the
+ * one-block k_bc kernel. The boundary kernel of a call's first step evaluates that step's drive; without boundary links a
+ * one-warp kernel does. */
 int cs_step(const cs_step_desc* d, int32_t a, int32_t steps, void* stream);
+int cs_step_ex(const cs_step_desc* d, const cs_step_layout* layout, int32_t a, int32_t steps, void* stream);
 
 /* Check a descriptor (HOST struct) as cs_step does, without launching anything. */
 int cs_step_check(const cs_step_desc* d);
@@ -246,6 +252,8 @@ int cs_step_check(const cs_step_desc* d);
 /* Capture `steps` steps starting from buffer a into a CUDA graph (lbm.py:436-442); *graph receives an opaque
  * handle for cs_graph_launch / cs_graph_destroy. The stream must not be the legacy default stream. */
 int cs_graph_capture(const cs_step_desc* d, int32_t a, int32_t steps, void* stream, void** graph);
+int cs_graph_capture_ex(const cs_step_desc* d, const cs_step_layout* layout, int32_t a, int32_t steps, void* stream,
+                        void** graph);
 
 /* ---------------------------------------------------------------------------------------------------------------
  * Batched step — many independent lattices (vessels of different sizes, clots and drives) advanced together. The
@@ -271,9 +279,13 @@ typedef struct cs_batch_desc {
                                            the bulk kernels' work counters (the boundary kernels reset them) */
 } cs_batch_desc;
 
-/* Enqueue `steps` batched steps; the first reads buffer a ^ parity[i] of instance i. */
+/* Enqueue `steps` batched steps; the first reads buffer a ^ parity[i] of instance i. layouts: HOST array (n_inst), or
+ * null. */
 int cs_batch_step(const cs_batch_desc* b, int32_t a, int32_t steps, void* stream);
+int cs_batch_step_ex(const cs_batch_desc* b, const cs_step_layout* layouts, int32_t a, int32_t steps, void* stream);
 int cs_batch_graph_capture(const cs_batch_desc* b, int32_t a, int32_t steps, void* stream, void** graph);
+int cs_batch_graph_capture_ex(const cs_batch_desc* b, const cs_step_layout* layouts, int32_t a, int32_t steps, void* stream,
+                              void** graph);
 int cs_graph_launch(void* graph, void* stream);
 int cs_graph_destroy(void* graph);
 
@@ -313,7 +325,7 @@ int cs_last_error(char* buf, int32_t len);
 const char* cs_version(void);
 
 /* sizeof of the ABI structs, so that bindings can check their layout: which = 0 cs_opening, 1 cs_step_desc;
- * which = 2 returns CS_SEG_STRIDE, 3 sizeof(cs_batch_desc). */
+ * which = 2 returns CS_SEG_STRIDE, 3 sizeof(cs_batch_desc), 4 sizeof(cs_step_layout). */
 size_t cs_abi_sizeof(int32_t which);
 
 #ifdef __cplusplus

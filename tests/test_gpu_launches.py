@@ -36,11 +36,11 @@ def test_launches_of_a_call(steps):
     coupled = simulate.ArterySolver(lat, 0.02, flux, [0.0], 0.0, 0.1)
 
     def step(s):
-        d = s._desc()
-        return kernels(s, lambda st: lib.cs_step(ctypes.byref(d), s.cur, steps, st))
+        d, x = s._desc(), s._layout()
+        return kernels(s, lambda st: lib.cs_step_ex(ctypes.byref(d), ctypes.byref(x), s.cur, steps, st))
     assert step(plain) == 2 * steps            # boundary links, nodes
     assert step(coupled) == 3 * steps          # and the resistances
     assert step(periodic) == 1 + steps         # no boundary kernel that could evaluate the first drive
     b = batch.BatchSolver([plain, lbm.Solver(lat, 0.02)])
     b._refresh()
-    assert kernels(b, lambda st: lib.cs_batch_step(ctypes.byref(b.desc), b.cur, steps, st)) == 2 * steps
+    assert kernels(b, lambda st: lib.cs_batch_step_ex(ctypes.byref(b.desc), b._layouts, b.cur, steps, st)) == 2 * steps
