@@ -1076,11 +1076,13 @@ int validate(const cs_step_desc* d, const cs_step_layout* layout) {
     return CS_OK;
 }
 
-// One division of the SM's memory between L1 and shared memory for every kernel of a step. By default the driver picks
+// One division of the SM's memory between L1 and shared memory for every kernel of a single lattice's step. By default the driver picks
 // it by each kernel's own shared memory (none in the boundary kernel, 9 blocks x 4.6 KB in the bulk kernel), and an SM
 // that changes it between two kernels drains first: the next kernel's blocks then do not start under the last one's
 // (20 k-node cylinder 9.6 us a step, with one division 5.0; tilted pipe of 75 k nodes 12.6 and 8.4). 28 % is the 64 KB
-// that nine blocks of the bulk kernel need; half of it leaves room for seven (artery 88.6 against 86.5 us).
+// that nine blocks of the bulk kernel need; half of it leaves room for seven (artery 88.6 against 86.5 us). The batched
+// kernels keep the driver's choice: persistent grids that start under one another took 68.9 us a step against 54.1 on four
+// FP32 vessels of 100-400 k nodes, 71.0 against 60.0 on five of 150-250 k, and grids of a block an item the same.
 constexpr int CARVEOUT = 28;
 
 int set_carveout(const void* fn) {
@@ -1472,10 +1474,6 @@ int launch_batch(const cs_batch_desc* b, const cs_step_layout* layouts, int a, i
                    : b->storage == CS_STORE_BF16 ? pick_batch_model<CS_STORE_BF16>(*b, dense)
                                                  : pick_batch_model<CS_STORE_F32>(*b, dense);
     BatchFn bound = pick_batch_boundary(b->storage, false), bound_start = pick_batch_boundary(b->storage, true);
-    for (BatchFn fn : {bulk, bound, bound_start, BatchFn(k_bc_batch), BatchFn(k_clock_empty_batch)}) {
-        const int rc = set_carveout(reinterpret_cast<const void*>(fn));
-        if (rc != CS_OK) return rc;
-    }
     bool empty = false, every = !layouts;           // every: some instance has no place for the next step's drive
     for (int i = 0; i < b->n_inst; ++i) {
         empty = empty || b->descs[i].n == 0;
