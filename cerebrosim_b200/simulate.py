@@ -184,9 +184,10 @@ class Probes:
             self._buf = torch.zeros(2 * m, dtype=torch.float64, device=s.dev)
             self.psum, self.umax = self._buf[:m], self._buf[m:].view(torch.float32)[:m]
             self._host = torch.empty(2 * m, dtype=torch.float64, pin_memory=True)
+            self._read = torch.cuda.Event()
 
     def enqueue(self):
-        """Reduce the fields on the solver's stream and start the read-back; `values` has them once it has passed."""
+        """Reduce the fields on the solver's stream and start the read-back; `values` waits for it."""
         s = self.s
         with torch.cuda.device(s.dev), torch.cuda.stream(s.stream):
             check(_lib.load().cs_probe_gather(ctypes_void(s.rho.data_ptr()), ctypes_void(s.vel[s.cur].data_ptr()),
@@ -195,8 +196,10 @@ class Probes:
                                               ctypes_void(self.psum.data_ptr()), ctypes_void(self.umax.data_ptr()),
                                               ctypes_void(s.stream.cuda_stream)))
             self._host.copy_(self._buf, non_blocking=True)
+            self._read.record(s.stream)
 
     def values(self):
+        self._read.synchronize()
         host = self._host.numpy()
         m = len(host) // 2
         p = np.where(self.count > 0, host[:self.n] / np.maximum(self.count, 1), np.nan)
@@ -204,7 +207,6 @@ class Probes:
 
     def sample(self):
         self.enqueue()
-        self.s.stream.synchronize()
         return self.values()
 
 
@@ -273,9 +275,8 @@ def run_beats(s, steps_per_beat, beats, every, probes=None, cmap=None, frames=40
                 p_host.copy_(s.p_out, non_blocking=True)
         if deferred:
             probes.enqueue()
-        if coupled or deferred:
-            s.stream.synchronize()
         if coupled:
+            s.stream.synchronize()
             series["Q"].append(q_host.numpy().copy())
             series["p_open"].append(p_host.numpy()[:s.n_open].astype(float))
         if probes is not None:
