@@ -261,24 +261,30 @@ def run_beats(s, steps_per_beat, beats, every, probes=None, cmap=None, frames=40
     series = {"step": [], "Q": [], "p_open": [], "p_probe": [], "umax": []}
     out = {"t_step": [], "p": [], "u": []}
     total = beats * steps_per_beat
-    coupled, deferred = hasattr(s, "Qlast"), hasattr(probes, "enqueue")
-    # a sample's values come back behind the steps on their stream, and the host waits for them once
-    if coupled:
+    # a sample's values come back behind the steps on their stream, and the host waits for them once; of probes with a
+    # `sample` of their own, and of other solvers, they are asked for one by one
+    coupled = hasattr(s, "Qlast")
+    behind = isinstance(s, ArterySolver) and type(s.Qlast) is DeviceArray
+    deferred = probes is not None and getattr(probes.sample, "__func__", None) is Probes.sample
+    if behind:
         q_host = torch.empty_like(s.Qlast.tensor, device="cpu", pin_memory=True)
         p_host = torch.empty_like(s.p_out, device="cpu", pin_memory=True)
     while s.steps < total:
         s.run(every, chunk=every)
         series["step"].append(s.steps)
-        if coupled:
+        if behind:
             with torch.cuda.device(s.dev), torch.cuda.stream(s.stream):
                 q_host.copy_(s.Qlast.tensor, non_blocking=True)
                 p_host.copy_(s.p_out, non_blocking=True)
         if deferred:
             probes.enqueue()
-        if coupled:
+        if behind:
             s.stream.synchronize()
             series["Q"].append(q_host.numpy().copy())
             series["p_open"].append(p_host.numpy()[:s.n_open].astype(float))
+        elif coupled:
+            series["Q"].append(s.Qlast.numpy().copy())
+            series["p_open"].append(s.p_out.cpu().numpy()[:s.n_open].astype(float))
         if probes is not None:
             p, um = probes.values() if deferred else probes.sample()
             series["p_probe"].append(p)
