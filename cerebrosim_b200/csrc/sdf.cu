@@ -4,8 +4,8 @@
 // Per voxel p = origin + (i, j, k) dx: for each branch, the minimum over its segments of the round-cone distance
 // |p - (a + t ab)| - r(t) (t = the clamped projection of p on the segment, r interpolated linearly), cut by the flat
 // caps near its open ends (a half-space max within 2.5 cap radii); branches are joined by the polynomial smooth
-// minimum with blend radius `blend`. Negative inside the lumen. One thread per voxel, C order (k fastest); a block
-// works a brick of voxels with the segments that can be nearest there.
+// minimum with blend radius `blend`. Negative inside the lumen. C order (k fastest); a block works a brick of voxels, two
+// a thread, with the segments that can be nearest there.
 #include "cs_common.cuh"
 
 namespace cs {
@@ -46,20 +46,25 @@ __device__ __forceinline__ float smin(float a, float b, float k) {
 // r0, r1 at its ends: anywhere in the brick |p - q| - r lies in [D_k(c) - h - max(r0, r1), D_k(c) + h - min(r0, r1)]
 // (a distance to a segment changes by at most the way walked). A segment whose lower end lies above the least upper
 // end U of all segments of its branch is never the minimum. For a voxel p and a segment of half-length l and midpoint
-// m, |p - q| >= |p - m| - l. Each bound carries a margin of 1e-5 of the lengths that enter it, over a hundred times
-// the rounding of its own evaluation and of the distances it is compared with. A comparison with NaN keeps the segment.
+// m, |p - q| >= |p - m| - l. Each bound carries a margin of 1e-5 of the lengths that enter it (the coordinates and the
+// grid's origin, the distance, the segment's own length and radii), over a hundred times the rounding of its own
+// evaluation and of the distances it is compared with. A segment shorter than 1e-6 is projected on by a bounded divisor,
+// which can put the point taken for the nearest anywhere on it: 1e-6 more. A comparison with NaN keeps the segment.
 constexpr int BX = 8, BY = 8, BZ = 8, SDF_PER = 2;       // voxels a thread, BY / SDF_PER apart along y
 constexpr int SDF_THREADS = BX * BY * BZ / SDF_PER;
-constexpr float SDF_MARGIN = 1.0e-5f;
+constexpr float SDF_MARGIN = 1.0e-5f, SDF_TINY = 1.0e-6f;
 
-// Axis distance of point c from segment k of the packed centrelines.
-__device__ __forceinline__ float axis_distance(const SdfArgs& s, int k, float cx, float cy, float cz) {
+// Axis distance of point c from segment k of the packed centrelines; margin: of the bounds made from it.
+__device__ __forceinline__ float axis_distance(const SdfArgs& s, int k, float cx, float cy, float cz, float size, float r0,
+                                                float r1, float& margin) {
     const float ax = __ldg(s.pts + 3 * k), ay = __ldg(s.pts + 3 * k + 1), az = __ldg(s.pts + 3 * k + 2);
     const float bx = __ldg(s.pts + 3 * k + 3) - ax, by = __ldg(s.pts + 3 * k + 4) - ay, bz = __ldg(s.pts + 3 * k + 5) - az;
     const float qx = cx - ax, qy = cy - ay, qz = cz - az;
     const float t = fminf(fmaxf((qx * bx + qy * by + qz * bz) / fmaxf(bx * bx + by * by + bz * bz, 1.0e-12f), 0.0f), 1.0f);
     const float ex = qx - bx * t, ey = qy - by * t, ez = qz - bz * t;
-    return sqrtf(ex * ex + ey * ey + ez * ez);
+    const float dk = sqrtf(ex * ex + ey * ey + ez * ez);
+    margin = SDF_MARGIN * (size + dk + fabsf(bx) + fabsf(by) + fabsf(bz) + fmaxf(fabsf(r0), fabsf(r1))) + SDF_TINY;
+    return dk;
 }
 
 // vessel.py:195-199: distance of p to the round cone from a along b with radius r0 + dr t.
@@ -98,17 +103,18 @@ __global__ void __launch_bounds__(SDF_THREADS) k_sdf(const SdfArgs s, const IDX 
         const float cy = s.origin[1] + (float(y0) + 0.5f * float(BY - 1)) * s.dx;
         const float cz = s.origin[2] + (float(z0) + 0.5f * float(BZ - 1)) * s.dx;
         const float h = 0.5f * s.dx * sqrtf(float((BX - 1) * (BX - 1) + (BY - 1) * (BY - 1) + (BZ - 1) * (BZ - 1)));
-        const float size = fabsf(cx) + fabsf(cy) + fabsf(cz) + 4.0f * h;     // of the coordinates in the brick
+        const float size = fabsf(cx) + fabsf(cy) + fabsf(cz) + 4.0f * h + fabsf(s.origin[0]) + fabsf(s.origin[1]) +
+                           fabsf(s.origin[2]);          // of the coordinates in the brick and the sums that gave them
         for (int b = 0; b < s.nbranch; ++b) {
             const int s0 = __ldg(s.br_start + b), last = s0 + __ldg(s.br_count + b) - 1;
             // least upper bound over the branch's segments, and the segment that has it
-            float u_own = 3.0e38f, dk = 0.0f, r0 = 0.0f, r1 = 0.0f;
+            float u_own = 3.0e38f, dk = 0.0f, r0 = 0.0f, r1 = 0.0f, margin = 0.0f;
             int k_own = -1;
             for (int k = s0 + tid; k < last; k += SDF_THREADS) {
-                dk = axis_distance(s, k, cx, cy, cz);
                 r0 = __ldg(s.rad + k);
                 r1 = __ldg(s.rad + k + 1);
-                const float up = dk + h - fminf(r0, r1) + SDF_MARGIN * (size + dk + fmaxf(fabsf(r0), fabsf(r1)));
+                dk = axis_distance(s, k, cx, cy, cz, size, r0, r1, margin);
+                const float up = dk + h - fminf(r0, r1) + margin;
                 if (up < u_own) {
                     u_own = up;
                     k_own = k;
@@ -142,12 +148,11 @@ __global__ void __launch_bounds__(SDF_THREADS) k_sdf(const SdfArgs s, const IDX 
                 bool keep = false;
                 if (k < last) {
                     if (last - s0 > SDF_THREADS) {         // of a single chunk the first pass left them in registers
-                        dk = axis_distance(s, k, cx, cy, cz);
                         r0 = __ldg(s.rad + k);
                         r1 = __ldg(s.rad + k + 1);
+                        dk = axis_distance(s, k, cx, cy, cz, size, r0, r1, margin);
                     }
-                    const float rm = fmaxf(r0, r1);
-                    keep = !(dk - h - rm - SDF_MARGIN * (size + dk + fmaxf(fabsf(r0), fabsf(r1))) > u);
+                    keep = !(dk - h - fmaxf(r0, r1) - margin > u);
                 }
                 const unsigned mask = __ballot_sync(0xffffffffu, keep);
                 if (lane == 0) s_cnt[warp] = __popc(mask);
@@ -168,7 +173,6 @@ __global__ void __launch_bounds__(SDF_THREADS) k_sdf(const SdfArgs s, const IDX 
                     const float bx = __ldg(s.pts + 3 * k + 3) - ax, by = __ldg(s.pts + 3 * k + 4) - ay,
                                 bz = __ldg(s.pts + 3 * k + 5) - az;
                     const float b2 = bx * bx + by * by + bz * bz, half = 0.5f * sqrtf(b2);
-                    const float margin = SDF_MARGIN * (size + dk + 2.0f * half + fmaxf(fabsf(r0), fabsf(r1)));
                     s_seg[0][o] = make_float4(ax, ay, az, r0);
                     s_seg[1][o] = make_float4(bx, by, bz, r1 - r0);
                     s_mid[o] = make_float4(ax + 0.5f * bx, ay + 0.5f * by, az + 0.5f * bz,
