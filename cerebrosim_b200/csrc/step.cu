@@ -768,34 +768,38 @@ __device__ __forceinline__ void node_update(const StepArgs& d, int a, int32_t n,
         const float ddx_ = -(1.0f - om) * edx, ddy_ = -(1.0f - om) * edy, ddz_ = -(1.0f - om) * edz;
         const float trd = (ddx_ + ddy_ + ddz_) / 3.0f;
         // FP32: a pair's links differ only in the sign of what is odd in c, so both come from one evaluation, and without a
-        // body force its terms are zero and left out (75 k-node pipe 9.1 -> 7.3 us a step). The 16-bit formats keep the
-        // link-by-link sums: another rounding in 32 bits would move stored values by a unit of the 16-bit format.
+        // body force its terms are zero and left out (75 k-node pipe 8.3 -> 7.5 us a step). Rounded as spelled out: left to
+        // the compiler's contraction, with the equilibria rounded before the difference, the error against 64 bits was 3 %
+        // above the link-by-link sums' (velocity, rms over 48 runs); so it is the same (0.999, density 1.001). The 16-bit
+        // formats keep the link-by-link sums: another rounding in 32 bits would move stored values by a unit of the 16-bit
+        // format.
         if constexpr (ST == CS_STORE_F32) {
             const float ke = 1.0f - 0.5f * om, ko = 1.0f - 0.5f * om_m;
+            const float rest = __fmaf_rn(-1.5f, usq, dr);
             {
-                const float even = fk[0] - wgt(0) * (dr - 1.5f * usq);
-                float v = fk[0] - om * even;
+                float v = __fmaf_rn(-om, __fmaf_rn(-wgt(0), rest, fk[0]), fk[0]);
                 if constexpr (FORCE) v += ke * (wgt(0) * (-3.0f * uF));
-                Pop<ST>::st(fout, uint32_t(n), wgt(0), v + wgt(0) * 4.5f * (0.0f - trd));
+                Pop<ST>::st(fout, uint32_t(n), wgt(0), __fmaf_rn(wgt(0) * 4.5f, 0.0f - trd, v));
             }
             Unroll<0, 13>::run([&](auto pc) {
                 constexpr int I = 1 + 2 * decltype(pc)::value;
                 constexpr int O = Lat::opp(I);
                 constexpr int x = Lat::cx(I), y = Lat::cy(I), z = Lat::cz(I);
                 const float cv = float(x) * ux + float(y) * uy + float(z) * uz;
-                const float eqp = wgt(I) * (dr + 4.5f * cv * cv - 1.5f * usq);
-                const float eqm = wgt(I) * (3.0f * cv + t3 * cu3.template h3<I>());
-                const float psi = wgt(I) * 4.5f * (float(x * x) * ddx_ + float(y * y) * ddy_ + float(z * z) * ddz_ - trd);
-                const float even = 0.5f * (fk[I] + fk[O]) - eqp, odd = 0.5f * (fk[I] - fk[O]) - eqm;
-                float vi = fk[I] - om * even - om_m * odd, vo = fk[O] - om * even + om_m * odd;
+                const float pd = float(x * x) * ddx_ + float(y * y) * ddy_ + float(z * z) * ddz_ - trd;
+                const float even = __fmaf_rn(-wgt(I), __fmaf_rn(4.5f * cv, cv, rest), 0.5f * (fk[I] + fk[O]));
+                const float odd = __fmaf_rn(-wgt(I), __fmaf_rn(3.0f, cv, t3 * cu3.template h3<I>()), 0.5f * (fk[I] - fk[O]));
+                const float e2 = __fmaf_rn(om, even, -wgt(I) * 4.5f * pd);
+                float vi = fk[I] - __fmaf_rn(om_m, odd, e2);
+                float vo = fk[O] - __fmaf_rn(-om_m, odd, e2);
                 if constexpr (FORCE) {
                     const float cF = float(x) * Fx + float(y) * Fy + float(z) * Fz;
                     const float sp = wgt(I) * (9.0f * cv * cF - 3.0f * uF), sm = wgt(I) * 3.0f * cF;
                     vi = vi + ke * sp + ko * sm;
                     vo = vo + ke * sp - ko * sm;
                 }
-                Pop<ST>::st(fout, uint32_t(I) * NP + uint32_t(n), wgt(I), vi + psi);
-                Pop<ST>::st(fout, uint32_t(O) * NP + uint32_t(n), wgt(I), vo + psi);
+                Pop<ST>::st(fout, uint32_t(I) * NP + uint32_t(n), wgt(I), vi);
+                Pop<ST>::st(fout, uint32_t(O) * NP + uint32_t(n), wgt(I), vo);
             });
         } else {
             Unroll<0, Q>::run([&](auto ic) {
