@@ -113,3 +113,78 @@ def test_probe_sizes(sizes):
         else:
             assert np.isnan(p[k])
     assert umax == pytest.approx(np.linalg.norm(u[np.concatenate(idx)], axis=1).max(), rel=4 * 2.0 ** -23)
+
+
+@pytest.mark.parametrize("block", [32, 128, 256])
+@pytest.mark.parametrize("ends", [2, 8])
+def test_flux_of_several_ends(ends, block):
+    """Every open end's flow and relaxed pressure, with 1 cell in 3 and 1 in 5 measured by an end of its own choice (in
+    blocks of 32 more rows than k_bc holds in flight): the FP64 sum over the velocity field up to the rounding of 1e5
+    additions, and p' = p + alpha (R Q - pref - p) from it up to a few roundings."""
+    lat = pipe("open_pipe_R16_L96")
+    lat = dict(lat, n_outlets=max(ends, lat["n_outlets"]))
+    n = lbm.n_nodes(lat)
+    rng = np.random.default_rng(ends)
+    idx = np.concatenate([np.arange(0, n, 3), np.arange(1, n, 5)])
+    flux = {"idx": idx, "w": rng.uniform(-1, 1, size=(len(idx), 3)).astype(np.float32), "slot": rng.integers(0, ends, len(idx))}
+    R = np.concatenate([[0.0], rng.uniform(0.1, 1.0, ends - 1)]).astype(np.float32)
+    s = simulate.ArterySolver(lat, 0.02, flux, R, 0.001, 0.1, model="regularised", block=block)
+    s.set_drive([0.02])
+    s.run(6)
+    before = s.p_out64.cpu().numpy()[:ends]
+    s.run(1)
+    u = s.fields()[1].astype(np.float64)
+    terms = (u[idx] * flux["w"]).sum(1)
+    q, after = s.Qlast.numpy(), s.p_out64.cpu().numpy()[:ends]
+    assert after[0] == s.drv.item()
+    for k in range(ends):
+        t = terms[flux["slot"] == k]
+        assert abs(q[k] - t.sum()) <= 1e5 * 2.0 ** -53 * np.abs(t).sum()
+        if k:
+            want = before[k] + 0.1 * (float(R[k]) * q[k] - 0.001 - before[k])
+            assert abs(after[k] - want) <= 1e-14 and after[k] != before[k]
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16", "bf16"])
+def test_pulls_past_the_l2(storage):
+    """The pulls that go out of the caches first (both buffers within the L2) and the others give the same fields bit for
+    bit: rows so far apart that the same lattice counts as larger than the L2 choose the others."""
+    lat = pipe("open_pipe_R7_L33")
+    out = []
+    for stride in (None, 3 << 20):
+        s = lbm.Solver(lat, 0.02, model="regularised", storage=storage)
+        l2 = torch.cuda.get_device_properties(s.dev).L2_cache_size
+        if stride:
+            with torch.cuda.stream(s.stream):
+                s.f = [torch.zeros((lbm.Q, stride), dtype=f.dtype, device=s.dev)[:, :s.npad] for f in s.f]
+        assert (2 * lbm.Q * s.f[0].stride(0) * s.f[0].element_size() > l2) == bool(stride)
+        s.set_drive([0.03, 0.01, 0.0], period=50, ramp=10)
+        s.set_outlet_pressure([0.001])
+        s.run(60, chunk=20)
+        out.append(s.fields())
+    assert np.abs(out[0][1]).max() > 0
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("persistent", [True, False])
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+def test_batch_rows(storage, persistent):
+    """A batch of members with padded rows and rows back to back, of even and odd parity, gives each member's own run."""
+    lats = [pipe("open_pipe_R7_L33"), pipe()]
+
+    def members():
+        out = [lbm.Solver(lat, 0.02, model="regularised", storage=storage) for lat in lats]
+        for k, s in enumerate(out):
+            s.set_drive([0.02 + 0.01 * k, 0.01, 0.0], period=30, ramp=5)
+            s.run(3 + k)
+        return out
+    alone, together = members(), members()
+    for s in alone:
+        s.run(25, chunk=10)
+    with torch.cuda.stream(together[1].stream):
+        together[1].f, together[1].vel = ([t.contiguous() for t in ts] for ts in (together[1].f, together[1].vel))
+    b = batch.BatchSolver(together, persistent=persistent)
+    b.run(25, chunk=10)
+    b.synchronize()
+    for a, t in zip(alone, together):
+        assert all(np.array_equal(x, y) for x, y in zip(a.fields(), t.fields())) and a.fields()[1].any()
