@@ -767,12 +767,12 @@ __device__ __forceinline__ void node_update(const StepArgs& d, int a, int32_t n,
         const float om_m = 1.0f / (0.5f + d.magic / (1.0f / om - 0.5f));
         const float ddx_ = -(1.0f - om) * edx, ddy_ = -(1.0f - om) * edy, ddz_ = -(1.0f - om) * edz;
         const float trd = (ddx_ + ddy_ + ddz_) / 3.0f;
-        // FP32: a pair's links differ only in the sign of what is odd in c, so both come from one evaluation, and without a
-        // body force its terms are zero and left out (75 k-node pipe 8.3 -> 7.5 us a step). Rounded as spelled out: left to
-        // the compiler's contraction, with the equilibria rounded before the difference, the error against 64 bits was 3 %
-        // above the link-by-link sums' (velocity, rms over 48 runs); so it is the same (0.999, density 1.001). The 16-bit
-        // formats keep the link-by-link sums: another rounding in 32 bits would move stored values by a unit of the 16-bit
-        // format.
+        // FP32: a pair's links differ only in the sign of what is odd in c, so the half sum and the half difference of the two
+        // are relaxed apart and added at the end; without a body force its terms are zero and left out (75 k-node pipe 8.3
+        // -> 7.0 us a step, 222 k nodes with a force 16.6 -> 13.0). Rounded as spelled out: left to the compiler's
+        // contraction, with the equilibria rounded before the difference, the velocity's error against 64 bits was 1.03 of
+        // the link-by-link sums' (rms over 48 runs), so it is 0.95 (density 1.00). The 16-bit formats keep the link-by-link
+        // sums: another rounding in 32 bits would move stored values by a unit of the 16-bit format.
         if constexpr (ST == CS_STORE_F32) {
             const float ke = 1.0f - 0.5f * om, ko = 1.0f - 0.5f * om_m;
             const float rest = __fmaf_rn(-1.5f, usq, dr);
@@ -787,17 +787,16 @@ __device__ __forceinline__ void node_update(const StepArgs& d, int a, int32_t n,
                 constexpr int x = Lat::cx(I), y = Lat::cy(I), z = Lat::cz(I);
                 const float cv = float(x) * ux + float(y) * uy + float(z) * uz;
                 const float pd = float(x * x) * ddx_ + float(y * y) * ddy_ + float(z * z) * ddz_ - trd;
-                const float even = __fmaf_rn(-wgt(I), __fmaf_rn(4.5f * cv, cv, rest), 0.5f * (fk[I] + fk[O]));
-                const float odd = __fmaf_rn(-wgt(I), __fmaf_rn(3.0f, cv, t3 * cu3.template h3<I>()), 0.5f * (fk[I] - fk[O]));
-                const float e2 = __fmaf_rn(om, even, -wgt(I) * 4.5f * pd);
-                float vi = fk[I] - __fmaf_rn(om_m, odd, e2);
-                float vo = fk[O] - __fmaf_rn(-om_m, odd, e2);
+                const float hs = 0.5f * (fk[I] + fk[O]), hd = 0.5f * (fk[I] - fk[O]);
+                const float even = __fmaf_rn(-wgt(I), __fmaf_rn(4.5f * cv, cv, rest), hs);
+                const float odd = __fmaf_rn(-wgt(I), __fmaf_rn(3.0f, cv, t3 * cu3.template h3<I>()), hd);
+                float pe = __fmaf_rn(wgt(I) * 4.5f, pd, __fmaf_rn(-om, even, hs)), mo = __fmaf_rn(-om_m, odd, hd);
                 if constexpr (FORCE) {
                     const float cF = float(x) * Fx + float(y) * Fy + float(z) * Fz;
-                    const float sp = wgt(I) * (9.0f * cv * cF - 3.0f * uF), sm = wgt(I) * 3.0f * cF;
-                    vi = vi + ke * sp + ko * sm;
-                    vo = vo + ke * sp - ko * sm;
+                    pe = __fmaf_rn(ke, wgt(I) * __fmaf_rn(9.0f * cv, cF, -3.0f * uF), pe);
+                    mo = __fmaf_rn(ko, wgt(I) * 3.0f * cF, mo);
                 }
+                const float vi = pe + mo, vo = pe - mo;
                 Pop<ST>::st(fout, uint32_t(I) * NP + uint32_t(n), wgt(I), vi);
                 Pop<ST>::st(fout, uint32_t(O) * NP + uint32_t(n), wgt(I), vo);
             });
