@@ -583,7 +583,7 @@ def main():
                              "frac": achieved / peak, "peak_kind": peak_kind,
                              "traffic": tr * N if tr else None, "traffic_source": tr_source,
                              "bytes_per_update": bplu,
-                             "kernel": "one step = k_boundary + the bulk kernel (k_bulk_pair: two nodes per "
+                             "kernel": "one step = k_boundary + the bulk kernel (k_bulk_dense: one node per "
                                        "thread), timed together"},
                 "back_to_back": {"ms_per_step": b2b * 1e3, "value": world * N / b2b / 1e6, "unit": "MLUPS",
                                  "note": "the same steps in one call without flushing: steady state with L2 reuse"},

@@ -8,7 +8,7 @@
 //     with the second node, q >= 0.5 with the node's own population), half-way bounce-back, the velocity inlet with the
 //     drive, the pressure outlet with p_out and the previous velocity — and stores it in the ghost slot
 //     f_in[i * fstride + n + g] of the step's input buffer.
-//  2. k_bulk (k_bulk_dense: the regularised step without body force in blocks of <= 128 threads, 9 per SM) — one
+//  2. k_bulk (k_bulk_dense: the regularised step without body force in blocks of <= 128 threads, 8 or 9 per SM) — one
 //     thread per fluid node, C-ordered nodes, link-major populations (the reference's SoA layout).
 //     Every link is a plain pull f_in[i * fstride + links[i * n + node]] (a fluid source or a ghost slot), so the 27
 //     loads carry no branch and issue back to back; for each link the warp's 32 sources are mostly consecutive,
@@ -830,8 +830,9 @@ __device__ __forceinline__ void node_update(const StepArgs& d, int a, int32_t n,
 }
 
 // Block bx of a lattice's bulk grid (nodes bx * blockDim .. + blockDim - 1). Called by every thread of the block.
-// OPEN: the lattice may have open ends (n_open > 0); compiled apart for the kernels that lose by carrying their
-// reduction. clock: this block also advances the clock.
+// OPEN: the lattice may have open ends (n_open > 0); compiled apart for the kernels that lose by carrying their reduction
+// (cylinder 5.14 us a step against 5.07; batches of a block an item 59.4 against 55.4 on four FP32 vessels of 100-400 k
+// nodes, 97.3 against 92.0 on six FP16 ones). clock: this block also advances the clock.
 template <int ST, int MODEL, bool GAL, bool FORCE, bool OPEN, bool FIRST = false, bool EARLY = false>
 __device__ __forceinline__ void bulk_body(const StepArgs& d, const int a, const int bx, const bool clock) {
     const int32_t n0 = int32_t(bx) * int32_t(blockDim.x);
@@ -911,15 +912,18 @@ __global__ void __launch_bounds__(MAX_BLOCK, MIN_BLOCKS) k_bulk(const StepArgs d
 
 // The regularised step without a body force (every open vessel) in blocks of at most 128 threads, compiled for as many
 // of them per SM as hide the pulls' latency best: 8 at 64 registers in FP32 (artery 79.6 us a step against 80.5 for 9 at
-// 56, 190 k-node artery 9.9 against 10.6), 9 at 56 in the 16-bit formats (67.4 against 67.6). The batched kernel, whose
-// descriptor handling needs the registers, keeps 64. (One build with and without open ends: at 56 registers the one
-// without their reduction spills 28 bytes, this one 8, and takes 89 us a step on the artery against 86.)
+// 56, 190 k-node artery 9.9 against 10.6), 9 at 56 in the 16-bit formats (67.4 against 67.6). One build with and without
+// open ends: the FP32 one without their reduction spills 8 bytes (this one none), 18.2 us a step on the pipe against 17.9.
 //
-// FIRST: a step reads a population once, writes it to the other buffer, and a step later that copy is what is read: with
-// both buffers about as large as the L2, lines that have been read must go before lines just written. Loads marked so
-// take the 347 k-node FP32 pipe (75 MB) from 20.4 to 18.1 us a step, 522 k nodes (113 MB) from 29.4 to 27.2, 678 k nodes
-// in FP16 (73 MB) from 31.7 to 27.5. Past the L2 they lose the sectors that neighbouring warps share: 678 k nodes in FP32
-// (146 MB) 36.4 to 37.5, the artery (322 MB) 79.6 to 86.1. So the line is the L2's size.
+// FIRST: a step reads a population once, writes it to the other buffer, and a step later that copy is what is read. While
+// both buffers fit the L2, lines that have been read should go before lines just written. Loads marked evict-first take
+// the 347 k-node FP32 pipe (75 MB) from 20.4 to 18.1 us a step, 522 k nodes (113 MB) from 29.4 to 27.2, 678 k nodes in FP16
+// (73 MB) from 31.7 to 27.5. The qualifier names the L1; that the gain is the L2's shows in DRAM reads (pipe: 12.8 MB a
+// step without it, 1.3 with it) and in that an L2 policy does the same (18.0 us; L1::no_allocate 17.9). Past the L2 they
+// lose the sectors that neighbouring warps share: 678 k nodes in FP32 (146 MB) 36.4 to 37.5, the artery (322 MB) 79.6 to
+// 86.1. So the line is the L2's size, of one lattice: several that run at once share it, which costs the concurrent
+// schedules 1-2 % on two streams and 3-6 % on four (four FP32 vessels of 300-340 k nodes 73.7 to 78.3 us a step), while one
+// after the other they gain as above (68.9 to 62.2).
 constexpr int DENSE_BLOCK = 128;
 constexpr int dense_blocks(int st) { return st == CS_STORE_F32 ? 8 : 9; }
 
@@ -931,8 +935,8 @@ __global__ void __launch_bounds__(DENSE_BLOCK, dense_blocks(ST)) k_bulk_dense(co
 // ---- 3. outlet resistances ----------------------------------------------------------------------------------------
 constexpr int BC_THREADS = 512;
 
-// simulate.py:76-82 in FP64 (one block of BC_THREADS threads); the drive of this step was stored by the boundary
-// kernel. Q_k = the flux blocks' partial sums: a thread adds its rows (all open ends of a row lie side by side), warps
+// simulate.py:76-82 in FP64 (one block of BC_THREADS threads); the drive of this step was stored by the bulk kernel's
+// clock block. Q_k = the flux blocks' partial sums: a thread adds its rows (all open ends of a row lie side by side), warps
 // reduce by shuffles and the warps' sums are added in order (the same order at every step and run). The kernel is pure
 // latency on the path from one step to the next: launched programmatically, it reads fb_list before the bulk kernel has
 // ended and lets the next boundary kernel become resident while it works. A tree over all threads per open end and an
@@ -1347,8 +1351,9 @@ __global__ void __launch_bounds__(MAX_BLOCK, MIN_BLOCKS) k_bulk_batch(const __gr
 }
 
 // One block per bulk item, no loop and no claims (grid_bulk = 0): the regularised step without body force in blocks
-// of at most 128 threads, compiled like k_bulk_dense for 9 blocks per SM, which the persistent loop's state does not
-// leave registers for. The block finds its instance by a binary search over the item prefix in the parameters.
+// of at most 128 threads, compiled for 9 blocks per SM in every format (FP32 too: 55.4 us a step against 57.6 for 8 on four
+// vessels of 100-400 k nodes), which the persistent loop's state does not leave registers for (at 56 it spills and loses
+// 9 %). The block finds its instance by a binary search over the item prefix in the parameters.
 template <int ST, bool GAL, bool OPEN>
 __global__ void __launch_bounds__(DENSE_BLOCK, 9) k_bulk_batch_dense(const __grid_constant__ BatchGroup g,
                                                                                   const int a) {
