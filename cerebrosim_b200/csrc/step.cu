@@ -426,9 +426,11 @@ __device__ __forceinline__ void store_regularised(void* fout, uint32_t NP, int32
 // The clock. A step reads its drive, drive2[a], from memory: evaluating it (coefficients from memory, a sine and a
 // cosine per harmonic) took about 4 us on the step's critical path, in the boundary kernel that everything waits for.
 // The bulk kernel of the step before evaluates it beside its nodes. Before the first step of a call there is none: its
-// boundary kernel (START) evaluates the drive, each warp for itself, and k_clock where there are no boundary links. (A
-// k_clock of its own before every call was a third launch of calls of one step: 41.4 us against 37.7 without.) A caller
-// without a drive2 has no place for the next step's drive, and every step begins like the first.
+// boundary kernel (START) evaluates the drive, each warp with an inlet link for itself and one for everybody, and k_clock
+// where there are no boundary links. (A k_clock of its own before every call was a third launch of calls of one step:
+// 41.4 us against 37.7 without. Evaluated by every warp, before its populations are asked for, it made a single step from a
+// cold L2 2 us longer on the 347 k-node pipe and 5 us on the 1.57 M-node artery.) A caller without a drive2 has no place for
+// the next step's drive, and every step begins like the first.
 __device__ __forceinline__ void advance_clock(const StepArgs& d, const int a) {
     const int t = d.tick[a];
     if (d.drive2) {
@@ -467,15 +469,13 @@ __device__ __forceinline__ void boundary_body(const StepArgs& d, const int a, co
     const bool live = g < d.gmax;
     Waited t;
     int32_t node, info;
-    float q, dv = 0.0f;
+    float q;
     if constexpr (START) {
         t = grid_dependency_wait();
         launch_dependents();
         node = live ? ld_step(t, d.gnode + slot) : -1;
         info = live ? ld_step(t, d.ginfo + slot) : 0;
         q = live ? ld_step(t, d.gq + slot) : 0.0f;
-        dv = drive_value_warp(d, d.tick[a]);
-        if (publish && threadIdx.x == 0) *d.drive_slot(a) = dv;
     } else {
         node = live ? __ldg(d.gnode + slot) : -1;
         info = live ? __ldg(d.ginfo + slot) : 0;
@@ -487,17 +487,30 @@ __device__ __forceinline__ void boundary_body(const StepArgs& d, const int a, co
     const bool second = info >= 0 && q < 0.5f;
     const uint32_t other = second ? uint32_t(io) * NP + uint32_t(info) : uint32_t(i) * NP + uint32_t(node);
     const float w = weight_rt(i);                                             // the opposite's weight too
-    if constexpr (!START) {
+    const void* fin = d.f[a];
+    float fo = 0.0f, f2 = 0.0f, dv = 0.0f;
+    if constexpr (START) {
+        if (node >= 0) {
+            fo = Pop<ST>::ld(t, fin, own, w);
+            f2 = Pop<ST>::ld(t, fin, other, w);
+        }
+        asm volatile("" ::"f"(fo), "f"(f2));                // in flight before the drive is evaluated
+        const bool first = publish && threadIdx.x < 32;
+        if (__any_sync(0xffffffffu, first || (node >= 0 && info == CS_INLET))) {
+            dv = drive_value_warp(d, d.tick[a]);
+            if (first && threadIdx.x == 0) *d.drive_slot(a) = dv;
+        }
+        if (node < 0) return;                               // padding slot of a direction with fewer links
+    } else {
         t = grid_dependency_wait();
         launch_dependents();                                // the bulk kernel may start its static loads
+        if (node < 0) return;
+        fo = Pop<ST>::ld(t, fin, own, w);
+        if (info >= CS_WALL) f2 = Pop<ST>::ld(t, fin, other, w);
     }
-    if (node < 0) return;                                   // padding slot of a direction with fewer links
-    const void* fin = d.f[a];
-    const float fo = Pop<ST>::ld(t, fin, own, w);
     float v;
     if (info >= CS_WALL) {
         // lbm.py:163-173: interpolated bounce-back, or half-way bounce-back without Bouzidi
-        const float f2 = Pop<ST>::ld(t, fin, other, w);
         v = fo;
         if (d.bouzidi) {
             if (q < 0.5f) {
